@@ -1,10 +1,10 @@
 // Limb-plane bookkeeping and per-entry MPF arithmetic on CUDA cores.
 //
-// All of these are HBM-bound streams over limb planes X[k*B + e]: one thread per entry, limb k of
-// consecutive entries adjacent in memory, so every load/store of a warp is one coalesced 128-byte
-// transaction.  Semantics follow sdpvibe/limbops.py and the CUDA strings of sdpvibe/mpf.py exactly.
+// All of these are streams over limb planes X[k*B + e]: one thread per entry, limb k of consecutive entries
+// adjacent in memory, so every load/store of a warp is one coalesced 128-byte transaction; the MPF operations
+// work on shared-memory columns (mpcol.cuh).  Semantics follow sdpvibe/limbops.py and the CUDA strings of sdpvibe/mpf.py exactly.
 #include "common.cuh"
-#include "mpcore.cuh"
+#include "mpcol.cuh"
 
 namespace {
 using namespace sdpv;
@@ -117,62 +117,40 @@ __global__ void badd_align_kernel(const int32_t* __restrict__ A, const int32_t* 
 }
 
 // ------------------------------------------------------------------ MPF (one exponent per entry)
-template <int LMAX>
-__global__ void mpf_mul_kernel(int L, i64 n, const int32_t* __restrict__ A, const i64* __restrict__ eA,
-                               const int32_t* __restrict__ Bm, const i64* __restrict__ eB, int bscalar,
-                               int32_t* __restrict__ O, i64* __restrict__ eO) {
-  i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+// One thread per entry, its words in shared-memory columns (mpcol.cuh).  Dynamic shared memory: 128 columns.
+__global__ void __launch_bounds__(kColThreads)
+    mpf_mul_kernel(int L, i64 n, const int32_t* __restrict__ A, const i64* __restrict__ eA,
+                   const int32_t* __restrict__ Bm, const i64* __restrict__ eB, int bscalar, int32_t* __restrict__ O,
+                   i64* __restrict__ eO) {
+  extern __shared__ u32 cols[];
+  const i64 i = (i64)blockIdx.x * kColThreads + threadIdx.x;
   if (i >= n) return;
-  i64 ib = bscalar ? 0 : i, nbn = bscalar ? 1 : n;
-  u32 a[LMAX], b[LMAX], r[LMAX];
-  for (int k = 0; k < L; k++) {
-    a[k] = (u32)A[(i64)k * n + i];
-    b[k] = (u32)Bm[(i64)k * nbn + ib];
-  }
-  i64 er;
-  mpf_mul_dev<LMAX>(a, eA[i], b, eB[ib], L, r, er);
-  for (int k = 0; k < L; k++) O[(i64)k * n + i] = (int32_t)r[k];
-  eO[i] = er;
+  const i64 ib = bscalar ? 0 : i, nbn = bscalar ? 1 : n;
+  col_mpf_mul(cols + threadIdx.x, A + i, n, eA[i], Bm + ib, nbn, eB[ib], L, O + i, n, eO + i);
 }
 
-template <int LMAX>
-__global__ void mpf_add_kernel(int L, i64 n, const int32_t* A, const i64* eA,
-                               const int32_t* __restrict__ Bm, const i64* __restrict__ eB, int sgn,
-                               int32_t* O, i64* eO, const int32_t* __restrict__ pred) {
-  i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kColThreads)
+    mpf_add_kernel(int L, i64 n, const int32_t* A, const i64* eA, const int32_t* Bm, const i64* eB, int sgn,
+                   int32_t* O, i64* eO, const int32_t* __restrict__ pred) {
+  extern __shared__ u32 cols[];
+  const i64 i = (i64)blockIdx.x * kColThreads + threadIdx.x;
   if (i >= n) return;
   if (pred && *pred == 0) return;                      // predicated launch: O / eO untouched
-  u32 a[LMAX], b[LMAX], r[LMAX];
-  for (int k = 0; k < L; k++) {
-    a[k] = (u32)A[(i64)k * n + i];
-    b[k] = (u32)Bm[(i64)k * n + i];
-  }
-  i64 er;
-  mpf_add_dev<LMAX>(a, eA[i], b, eB[i], sgn, L, r, er);
-  for (int k = 0; k < L; k++) O[(i64)k * n + i] = (int32_t)r[k];
-  eO[i] = er;
+  col_mpf_add(cols + threadIdx.x, A + i, n, eA[i], Bm + i, n, eB[i], sgn, L, O + i, n, eO + i);
 }
 
-template <int LMAX>
-__global__ void mpf_norm_kernel(int L, int LI, i64 n, const int32_t* __restrict__ X, const i64* __restrict__ eI,
-                                int32_t* __restrict__ O, i64* __restrict__ eO) {
-  i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kColThreads)
+    mpf_norm_kernel(int L, int LI, i64 n, const int32_t* __restrict__ X, const i64* __restrict__ eI,
+                    int32_t* __restrict__ O, i64* __restrict__ eO) {
+  extern __shared__ u32 cols[];
+  const i64 i = (i64)blockIdx.x * kColThreads + threadIdx.x;
   if (i >= n) return;
-  u32 w[160], r[LMAX];
-  for (int k = 0; k < LI; k++) w[k] = (u32)X[(i64)k * n + i];
-  bool ng = w[LI - 1] >> 31;
-  if (ng) neg_words(w, LI);
-  int bl = bitlen_mag(w, LI);
-  if (!bl) {
-    for (int k = 0; k < L; k++) O[(i64)k * n + i] = 0;
-    eO[i] = SDPV_EZ;
-    return;
-  }
-  int s = bl - (32 * L - 2);
-  mag_shift(w, LI, s, r, L);
-  if (ng) neg_words(r, L);
-  for (int k = 0; k < L; k++) O[(i64)k * n + i] = (int32_t)r[k];
-  eO[i] = eI[i] + s;
+  u32* c = cols + threadIdx.x;
+  col_stage(c, X + i, n, LI);
+  cp_async_commit();
+  const i64 ei = eI[i];
+  cp_async_wait<0>();
+  col_mpf_norm(c, LI, ei, L, O + i, n, eO + i);
 }
 
 // float64 -> normalised MPF, exactly: the 53-bit significand (subnormals included) shifted to NB = 32L-2 bits
@@ -219,14 +197,32 @@ __global__ void from_f64_kernel(int L, i64 n, const double* __restrict__ V, int3
 
 inline unsigned blocks(i64 n) { return (unsigned)((n + kThreads - 1) / kThreads); }
 
-#define SDPV_LMAX_DISPATCH(L, KERNEL, ...)                                     \
-  do {                                                                         \
-    if ((L) <= 8) KERNEL<8><<<blocks(n), kThreads, 0, st>>>(__VA_ARGS__);      \
-    else if ((L) <= 16) KERNEL<16><<<blocks(n), kThreads, 0, st>>>(__VA_ARGS__); \
-    else if ((L) <= 32) KERNEL<32><<<blocks(n), kThreads, 0, st>>>(__VA_ARGS__); \
-    else if ((L) <= 64) KERNEL<64><<<blocks(n), kThreads, 0, st>>>(__VA_ARGS__); \
-    else KERNEL<160><<<blocks(n), kThreads, 0, st>>>(__VA_ARGS__);             \
-  } while (0)
+inline unsigned col_blocks(i64 n) { return (unsigned)((n + kColThreads - 1) / kColThreads); }
+
+// Columns of `words` words for a CTA; the kernel's shared-memory limit is raised to the largest call's (160
+// limbs), once per device.
+template <class Kernel>
+int col_smem(Kernel kernel, int words, int most, bool (&set)[64], size_t& smem) {
+  smem = (size_t)words * kColThreads * 4;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!set[dev & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most * kColThreads * 4);
+    if (e != cudaSuccess) return sdpv::set_cuda_error(e);
+    set[dev & 63] = true;
+  }
+  return SDPV_OK;
+}
+
+int launch_add(int L, i64 n, const int32_t* A, const i64* eA, const int32_t* Bm, const i64* eB, int sgn, int32_t* O,
+               i64* eO, const int32_t* pred, cudaStream_t st) {
+  static bool set[64] = {};
+  size_t smem;
+  const int rc = col_smem(mpf_add_kernel, 2 * L + 2, 2 * 160 + 2, set, smem);
+  if (rc != SDPV_OK) return rc;
+  mpf_add_kernel<<<col_blocks(n), kColThreads, smem, st>>>(L, n, A, eA, Bm, eB, sgn, O, eO, pred);
+  return sdpv::launch_status();
+}
 
 }  // namespace
 
@@ -269,8 +265,11 @@ extern "C" int sdpv_mpf_mul(int L, int64_t n, const int32_t* A, const int64_t* e
                             const int64_t* eB, int bscalar, int32_t* O, int64_t* eO, void* stream) {
   if (L < 1 || L > 160 || n < 0) return SDPV_EINVAL;
   if (n == 0) return SDPV_OK;
-  cudaStream_t st = sdpv::as_stream(stream);
-  SDPV_LMAX_DISPATCH(L, mpf_mul_kernel, L, n, A, eA, Bm, eB, bscalar, O, eO);
+  static bool set[64] = {};
+  size_t smem;
+  const int rc = col_smem(mpf_mul_kernel, 2 * ((L + 3) & ~3), 2 * 160, set, smem);
+  if (rc != SDPV_OK) return rc;
+  mpf_mul_kernel<<<col_blocks(n), kColThreads, smem, sdpv::as_stream(stream)>>>(L, n, A, eA, Bm, eB, bscalar, O, eO);
   return sdpv::launch_status();
 }
 
@@ -278,9 +277,7 @@ extern "C" int sdpv_mpf_add(int L, int64_t n, const int32_t* A, const int64_t* e
                             const int64_t* eB, int sgn, int32_t* O, int64_t* eO, void* stream) {
   if (L < 1 || L > 160 || n < 0) return SDPV_EINVAL;
   if (n == 0) return SDPV_OK;
-  cudaStream_t st = sdpv::as_stream(stream);
-  SDPV_LMAX_DISPATCH(L, mpf_add_kernel, L, n, A, eA, Bm, eB, sgn, O, eO, (const int32_t*)nullptr);
-  return sdpv::launch_status();
+  return launch_add(L, n, A, eA, Bm, eB, sgn, O, eO, nullptr, sdpv::as_stream(stream));
 }
 
 extern "C" int sdpv_mpf_add_if(int L, int64_t n, const int32_t* A, const int64_t* eA, const int32_t* Bm,
@@ -288,9 +285,7 @@ extern "C" int sdpv_mpf_add_if(int L, int64_t n, const int32_t* A, const int64_t
                                void* stream) {
   if (L < 1 || L > 160 || n < 0 || !pred) return SDPV_EINVAL;
   if (n == 0) return SDPV_OK;
-  cudaStream_t st = sdpv::as_stream(stream);
-  SDPV_LMAX_DISPATCH(L, mpf_add_kernel, L, n, A, eA, Bm, eB, sgn, O, eO, pred);
-  return sdpv::launch_status();
+  return launch_add(L, n, A, eA, Bm, eB, sgn, O, eO, pred, sdpv::as_stream(stream));
 }
 
 extern "C" int sdpv_mpf_from_f64(int L, int64_t n, const double* V, int32_t* O, int64_t* eO, void* stream) {
@@ -304,7 +299,10 @@ extern "C" int sdpv_mpf_norm(int L, int LI, int64_t n, const int32_t* X, const i
                              int64_t* eO, void* stream) {
   if (L < 1 || L > 160 || LI < 1 || LI > 160 || n < 0) return SDPV_EINVAL;
   if (n == 0) return SDPV_OK;
-  cudaStream_t st = sdpv::as_stream(stream);
-  SDPV_LMAX_DISPATCH(L, mpf_norm_kernel, L, LI, n, X, eI, O, eO);
+  static bool set[64] = {};
+  size_t smem;
+  const int rc = col_smem(mpf_norm_kernel, LI, 160, set, smem);
+  if (rc != SDPV_OK) return rc;
+  mpf_norm_kernel<<<col_blocks(n), kColThreads, smem, sdpv::as_stream(stream)>>>(L, LI, n, X, eI, O, eO);
   return sdpv::launch_status();
 }
