@@ -30,24 +30,31 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn encode_tiled_fn();
 
+// Per modulus: m, (M/m)^-1 mod m, float(inv / m), 0x4B400000 m mod 2^32 (the bits of 1.5 2^23 times m).
+struct __align__(16) CrtMod {
+  int32_t m, inv;
+  float invm;
+  int32_t cm;
+};
+
 // Device-side RNS tables of one limb count (see ctx.cu).
 struct CtxDev {
   int L, n, E, W;
   int npad;          // moduli rounded up to 128 (MMA M of the decomposition)
   int kt;            // 128-byte K tiles of the byte-by-table product (ceil(4L/128))
   int npad16;        // moduli rounded up to 32 bytes (K of the CRT digit product, in 128-byte tiles)
-  int Epad;          // CRT digits rounded up to 128 (N chunks of the digit product)
+  int Epad;          // CRT digit rows (4 + E) rounded up to 128 (N chunks of the digit product)
   int32_t* mods;     // (n)
   float* minv;       // (n) float(1/m)
   int32_t* c14;      // (n) 2^14 mod m
   int32_t* c1;       // (n) C1 (sdpvibe/rns.py:183)
   int32_t* c1m2;     // (n) C1 - C2 (top limb negative)
-  int32_t* inv;      // (n) (M/m)^-1 mod m
-  int32_t* md;       // (Epad) signed base-256 digits of M, zero padded
+  CrtMod* crtmod;    // (128 ktc) the CRT pre-pass's constants per modulus, zeros past n
+  u32* negm;         // (W) words of 2^(8E) - M
   uint8_t* tab;      // decomposition tables as swizzled SMEM images: [group][lo|hi][kt][128 rows][128 B]
   uint8_t* tabu;     // the same layout with unsigned digits of the canonical 256^j mod m (hi = t >> 7,
                      // lo = t & 127) and column 4L = (-2^(32L)) mod m against the sign byte
-  uint8_t* ct;       // CRT digit table as swizzled SMEM images: [chunk][ktc][128 rows][128 B]
+  uint8_t* ct;       // CRT digit table as swizzled SMEM images: [chunk][yh | yl][ktc][128 rows][128 B]
   int ktc;           // 128-byte K tiles of the CRT product (ceil(n/128))
 };
 

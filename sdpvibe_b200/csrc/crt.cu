@@ -1,200 +1,237 @@
 // CRT reconstruction fused with rounding.
 //
 // For an entry with residues a_i (n moduli m_i, M = prod m_i, |value| < M/4):
-//   y_i = a_i (M/m_i)^-1 mod m_i  (centred),  k = round(sum y_i / m_i),
-//   value = sum_i y_i (M/m_i) - k M = sum_t (Z_t - k Md_t) 256^t,  Z_t = sum_i Ct[t][i] y_i
-// with Ct[t][i] the signed base-256 digits of M/m_i (sdpvibe/rns.py:140-159, 227-245;
-// sdpvibe/limbops.py:85-152).  A CTA handles one or two tiles of 128 entries; each tile goes through:
-//   * pre-pass (one thread per entry): y_i from the int16 accumulator, split y = 128 yh + yl into
-//     two K-major int8 tiles in shared memory, and k;
-//   * digit contraction on the tensor cores, 64 digits at a time: Zh = Yh Ct^T, Zl = Yl Ct^T
-//     (tcgen05.mma kind::i8, M = 128 entries, N = 64 digits, K = moduli), Ct resident in shared memory;
-//   * epilogue (the same thread, TMEM lane = entry): z = 128 Zh + Zl - k Md, carried into 32-bit words;
-//     then either the words + bit length (crt_block) or the MPF renormalisation of mpf_norm
-//     (magnitude rounded half up to NB = 32L-2 bits) written straight to the output limb planes.
+//   y_i = a_i (M/m_i)^-1 mod m_i in [0, m_i),  k = round(sum y_i / m_i),
+//   value = sum_i y_i (M/m_i) - k M  (sdpvibe/rns.py:140-159, 227-245; sdpvibe/limbops.py:85-152).
+// One CTA of 128 threads per tile of 128 entries (persistent over tiles):
+//   * pre-pass (one thread per entry): y_i from the int16 accumulator, its digits y = 128 yh + yl as two
+//     K-major byte rows in shared memory;
+//   * digit contraction on the tensor cores: Z = [Yh Yl] C^T (tcgen05.mma kind::i8 on unsigned bytes, M = 128
+//     entries, N = 128 digit rows per chunk, K = both digits of every modulus), C = the base-256 digits of 128
+//     M/m_i and M/m_i, preceded by four rows that give sum y_i round(2^29 / m_i), i.e. k (ctx.cu).  All chunks
+//     are issued back to back into TMEM (one column per digit) and waited for once;
+//   * epilogue (the same thread, TMEM lane = entry): a word is z0 + 2^8 z1 + 2^16 z2 + 2^24 z3 + k N_w + carry
+//     with N = 2^(32W) - M, all of it off the carry chain but one 64-bit add;
+//   * crt_block streams the words out; crt_norm puts them in the thread's column of the tile that held Y (the
+//     products are done with it) and renormalises from there (mpcol.cuh).
 // No intermediate leaves the SM; one launch replaces crt_pre + digit GEMM + crt_carry + normalize.
+//
+// What bounds it: instruction issue of the pre-pass (about 11 instructions per residue) and, for a few tiles,
+// the latency of one tile's phases.  Both digits of y in one contraction halve the TMEM columns and take the
+// digit recombination and k Md out of the epilogue.  Measured (B200, against two signed digit products in four
+// waited-for chunks with the words in local memory): 158760 entries at 116 moduli 130 -> 68 us, 65536 at 104
+// 48 -> 30 us, 1000 entries 37 -> 15 us; crt_block of 1024 entries 22 -> 15 us.  Two CTAs per SM, one tile each
+// (102 KB at 116 moduli): the table twice on the SM costs less than two tiles waiting for one another.
 #include "common.cuh"
-#include "mpcore.cuh"
+#include "mpcol.cuh"
 
 namespace {
 using namespace sdpv;
 
-constexpr int kThreads = 128;              // per 128-entry tile (TPC tiles per CTA: 128 TPC threads)
-constexpr int kDig = 64;                    // digits per MMA chunk (N)
+constexpr int kThreads = kColThreads;       // = entries of a tile
+constexpr int kDig = 128;                   // digit rows per chunk (N)
 constexpr u32 kSlice = 128 * 128;
+constexpr int kNmax = 256;                  // moduli: two 128-byte K tiles per digit plane
+constexpr int kWmax = 128;                  // words
+constexpr int kSlots = 4;                   // digit chunks (512 TMEM columns), and table slots, at most
+constexpr size_t kHead = 6144;              // barriers, CrtMod[kNmax], N[kWmax]
 
-struct CrtSmemHead {
-  u64 bar_ct, bar_mma[2];
+struct CrtHead {
+  u64 full[kSlots], empty[kSlots], done;
   u32 tmem_slot;
   int abort;
 };
 
-constexpr int kNmax = 320;                  // moduli tables staged in shared memory (n <= 320)
-constexpr int kEmax = 640;                  // CRT digits staged in shared memory (E <= 640)
-struct CrtTables {
-  int m[kNmax], inv[kNmax];
-  float minv[kNmax];
-  int md[kEmax];
-};
+// Four digit columns as one word's contribution.  WIDE: z0 + 2^8 z1 may exceed 32 bits (z <= n 381 255, so for
+// n > 168 as 257 n 381 255 >= 2^32).
+template <bool WIDE>
+__device__ __forceinline__ u64 digit_word(const u32* z) {
+  if (WIDE) return ((u64)z[0] + ((u64)z[1] << 8)) + ((((u64)z[2]) + ((u64)z[3] << 8)) << 16);
+  return (u64)(z[1] * 256u + z[0]) + (u64)(z[3] * 256u + z[2]) * 65536ull;
+}
 
-// Dynamic shared memory: [head (8 KB)] per tile [Yh: ktc slices] [Yl: ktc slices], then [Ct: Epad/128 * ktc
-// slices].  TPC tiles per CTA (1 or 2): with 2 the digit table Ct is staged once for two tiles, so two CTAs of
-// 2 x 128 entries fit an SM where three of 128 did (the tables, not the tiles, fill shared memory).
-template <int MODE, int TPC>
-__global__ void __launch_bounds__(kThreads * TPC)
+// Dynamic shared memory: [head] [Y: 2 ktc slices] [nslot chunk slots of 2 ktc slices].  The whole table stays
+// resident where it fits (n <= 128); else its chunks pass through the slots, from L2, once per tile.
+template <int MODE, bool WIDE>
+__global__ void __launch_bounds__(kThreads, 2)
     crt_kernel(const int16_t* __restrict__ acc, i64 ldg, i64 N, i64 j0, i64 w, i64 rows, i64 rows_per_block,
-               const int64_t* __restrict__ rowexp, const int64_t* __restrict__ colexp, int L, int n, int E, int W,
-               int ktc, int Epad, const int32_t* __restrict__ mods, const float* __restrict__ minvs,
-               const int32_t* __restrict__ invs, const int32_t* __restrict__ md, const uint8_t* __restrict__ ct,
-               int32_t* __restrict__ out, int64_t* __restrict__ out2, const int32_t* __restrict__ pred,
-               unsigned* __restrict__ err) {
+               const int64_t* __restrict__ rowexp, const int64_t* __restrict__ colexp, int L, int n, int W, int ktc,
+               int nchunk, int nslot, u32 tcols, const CrtMod* __restrict__ mods, const u32* __restrict__ negm,
+               const uint8_t* __restrict__ ct, int32_t* __restrict__ out, int64_t* __restrict__ out2,
+               const int32_t* __restrict__ pred, unsigned* __restrict__ err) {
   if (pred && *pred == 0) return;                      // predicated launch: nothing to do this time
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  CrtSmemHead& H = *reinterpret_cast<CrtSmemHead*>(base);
-  CrtTables& TB = *reinterpret_cast<CrtTables*>(base + 64);
-  const int tid = threadIdx.x, warp = tid >> 5, half = tid >> 7, lt = tid & 127;   // tile of the CTA, entry
-  uint8_t* Yh = base + 8192 + (size_t)half * 2 * ktc * kSlice;
+  CrtHead& H = *reinterpret_cast<CrtHead*>(base);
+  CrtMod* TB = reinterpret_cast<CrtMod*>(base + 1024);
+  u32* NM = reinterpret_cast<u32*>(base + 1024 + sizeof(CrtMod) * kNmax);
+  const int tid = threadIdx.x, warp = tid >> 5;
+  uint8_t* Yh = base + kHead;
   uint8_t* Yl = Yh + (size_t)ktc * kSlice;
-  uint8_t* Ct = base + 8192 + (size_t)TPC * 2 * ktc * kSlice;
+  u32* col = reinterpret_cast<u32*>(Yh) + tid;         // this entry's word column, once Y is free
+  const u32 cbytes = 2u * ktc * kSlice;                // one chunk of the table
+  uint8_t* slots = Yh + cbytes;
   const i64 B = rows * w;
   const i64 ntiles = (B + 127) / 128;
+  const bool resident = nslot >= nchunk;
+
+  i64 tile = blockIdx.x;
+  i64 e = tile * 128 + tid;
+  bool valid = e < B;
+  i64 r = valid ? e / w : 0, jj = valid ? e - r * w : 0;
+  const int16_t* ap = acc + r * N + j0 + jj;
+  // 32 residues at a time, the next 32 in flight while these are used (the first before any set-up)
+  auto load = [&](int gb, int (&v)[32]) {
+#pragma unroll
+    for (int q = 0; q < 32; q++) v[q] = (valid && gb + q < n) ? (int)__ldcs(ap + (i64)(gb + q) * ldg) : 0;
+  };
+  int va[32], vb[32];
+  load(0, va);
 
   if (tid == 0) {
-    mbar_init(&H.bar_ct, 1);
-    for (int h = 0; h < TPC; h++) mbar_init(&H.bar_mma[h], 1);
+    for (int s = 0; s < kSlots; s++) {
+      mbar_init(&H.full[s], 1);
+      mbar_init(&H.empty[s], 1);
+    }
+    mbar_init(&H.done, 1);
     H.abort = 0;
     mbar_fence_init();
+    for (int s = 0; s < nslot; s++) {                  // nslot <= nchunk
+      mbar_expect_tx(&H.full[s], cbytes);
+      for (u32 o = 0; o < cbytes; o += kSlice) bulk_load(slots + s * cbytes + o, ct + (size_t)s * cbytes + o, kSlice, &H.full[s]);
+    }
   }
   if (warp == 0) {
-    tmem_alloc(&H.tmem_slot, 2 * kDig * TPC);
+    tmem_alloc(&H.tmem_slot, tcols);
     tmem_relinquish();
   }
-  for (int g = tid; g < kNmax; g += kThreads * TPC) {
-    TB.m[g] = g < n ? mods[g] : 1;
-    TB.inv[g] = g < n ? invs[g] : 0;
-    TB.minv[g] = g < n ? minvs[g] : 1.f;
-  }
-  for (int t = tid; t < kEmax; t += kThreads * TPC) TB.md[t] = t < E ? md[t] : 0;
+  for (int g = tid; g < 128 * ktc && g < kNmax; g += kThreads) TB[g] = mods[g];
+  for (int k = tid; k < W; k += kThreads) NM[k] = negm[k];
   __syncthreads();
   tc_fence_after();
-  const u32 tmem = H.tmem_slot + (u32)half * 2 * kDig;              // this tile's Zh, Zl columns
-  if (tid == 0) {
-    u32 bytes = (u32)(Epad / 128) * ktc * kSlice;
-    mbar_expect_tx(&H.bar_ct, bytes);
-    for (u32 off = 0; off < bytes; off += kSlice) bulk_load(Ct + off, ct + off, kSlice, &H.bar_ct);
-  }
-  if (!mbar_wait(&H.bar_ct, 0, err)) H.abort = 1;
-
-  const u32 idesc = idesc_i8(128, kDig);
+  const u32 tmem = H.tmem_slot;
+  const u32 lane0 = (u32)(warp * 32) << 16;
+  const u32 idesc = idesc_u8(128, kDig);
   const int ksteps = (n + 31) / 32;
-  const int nchunk = (E + kDig - 1) / kDig;
-  u32 phase = 0;
-  u32 words[160];
+  u32 seq = 0, phase = 0;                              // chunks used so far, parity of `done`
 
-  for (i64 tile2 = blockIdx.x; tile2 * TPC < ntiles && !H.abort; tile2 += gridDim.x) {
-    // ---- pre-pass: y_i, its int8 digits, k
-    const i64 tile = tile2 * TPC + half;
-    const i64 e = tile * 128 + lt;
-    const bool valid = e < B;
-    const i64 r = valid ? e / w : 0, jj = valid ? e - (e / w) * w : 0;
-    const int16_t* ap = acc + r * N + j0 + jj;
-    float ks = 0.f;
-    for (int gb = 0; gb < ktc * 128; gb += 64) {
-      // the 64 loads of this group of moduli issued before any is used (they are independent): the pre-pass
-      // is bound by memory latency, one per group
-      int av[64];
+  while (true) {
+    // ---- pre-pass: the digits of y_i
+    auto digits = [&](int gb, const int (&v)[32]) {
 #pragma unroll
-      for (int q = 0; q < 64; q++) av[q] = (valid && gb + q < n) ? (int)__ldcs(ap + (i64)(gb + q) * ldg) : 0;
-#pragma unroll
-      for (int h = 0; h < 4; h++) {                              // 16 moduli per 16-byte digit chunk
+      for (int h = 0; h < 2; h++) {                    // 16 moduli per 16-byte chunk
         u32 ph[4], pl[4];
 #pragma unroll
-        for (int q = 0; q < 16; q++) {
-          const int g = gb + 16 * h + q;
-          int y = 0;
-          if (valid && g < n) {
-            const int m = TB.m[g];
-            const float mi = TB.minv[g];
-            // centred residue of x = a inv (0 <= x < 2^30): nearest quotient from the float estimate (off by
-            // at most one), then at most one correction each way into [-(m >> 1), m >> 1]
-            const int x = av[16 * h + q] * TB.inv[g];
-            y = x - __float2int_rn(__int2float_rn(x) * mi) * m;
-            y -= (y > (m >> 1)) ? m : 0;
-            y += (y < -(m >> 1)) ? m : 0;
-            ks += (float)y * mi;
+        for (int q4 = 0; q4 < 4; q4++) {
+          u32 y[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            const int a = v[16 * h + 4 * q4 + u];
+            const int4 c = *reinterpret_cast<const int4*>(&TB[gb + 16 * h + 4 * q4 + u]);
+            // x = a inv, q = round(x / m) from the float product (off by less than 0.002): |x - q m| <= 0.502 m,
+            // so one correction gives y in [0, m)
+            const float fa = __int_as_float(0x4B008000 + a) - 8421376.0f;
+            const int qb = __float_as_int(fmaf(fa, __int_as_float(c.z), 12582912.0f));
+            const int x = a * c.y + c.w - qb * c.x;
+            y[u] = (u32)(x + ((x >> 31) & c.x));
           }
-          int yl = ((y + 64) & 127) - 64, yh = (y - yl) >> 7;
-          if ((q & 3) == 0) ph[q >> 2] = pl[q >> 2] = 0;
-          ph[q >> 2] |= (u32)(yh & 255) << (8 * (q & 3));
-          pl[q >> 2] |= (u32)(yl & 255) << (8 * (q & 3));
+          const u32 p01 = y[0] + (y[1] << 16), p23 = y[2] + (y[3] << 16);
+          ph[q4] = __byte_perm(p01 >> 7, p23 >> 7, 0x6420);
+          pl[q4] = __byte_perm(p01, p23, 0x6420) & 0x7F7F7F7Fu;
         }
-        const int g16 = gb + 16 * h;
-        int kt = g16 >> 7, chunk = (g16 & 127) >> 4;
-        *reinterpret_cast<uint4*>(Yh + kt * kSlice + sw128_off(lt, chunk)) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
-        *reinterpret_cast<uint4*>(Yl + kt * kSlice + sw128_off(lt, chunk)) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+        const int g16 = gb + 16 * h, kt = g16 >> 7, chunk = (g16 & 127) >> 4;
+        *reinterpret_cast<uint4*>(Yh + kt * kSlice + sw128_off(tid, chunk)) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
+        *reinterpret_cast<uint4*>(Yl + kt * kSlice + sw128_off(tid, chunk)) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
       }
+    };
+    for (int gb = 0; gb < n; gb += 64) {
+      if (gb + 32 < n) load(gb + 32, vb);
+      digits(gb, va);
+      if (gb + 32 >= n) break;
+      if (gb + 64 < n) load(gb + 64, va);
+      digits(gb + 32, vb);
     }
-    const i64 kq = (i64)__float2int_rd(ks + 0.5f);
-    const int kq32 = (int)kq;                                          // |k| <= n / 2
     fence_proxy_async_smem();
     __syncthreads();
 
-    // ---- digit chunks: MMA, then carry into words (crt_block streams them straight out, tracking the
-    //      highest word that differs from each possible sign extension for the bit length)
-    i64 carry = 0;
-    int nw = 0;
-    int hz = -1, ho = -1;                              // highest word != 0, != 0xffffffff
+    // ---- digit products, carried into words
+    u32 kq = 0, carry = 0;
+    int hz = -1, ho = -1;                              // crt_block: highest word != 0, != 0xffffffff
     u32 hzv = 0, hov = 0, wtop = 0;
-    for (int ch = 0; ch < nchunk; ch++) {
-      if (lt == 0) {                                   // one issuing thread per tile
-        tc_fence_after();
-        const u32 ctc = smem_u32(Ct) + (u32)((ch * kDig) / 128) * ktc * kSlice + (u32)((ch * kDig) % 128) * 128;
-        for (int s = 0; s < ksteps; s++) {
-          int kt = s >> 2, ko = (s & 3) * 32;
-          u64 bd = sdesc_sw128(ctc + kt * kSlice + ko);
-          mma_i8(tmem + 0, sdesc_sw128(smem_u32(Yh) + kt * kSlice + ko), bd, idesc, s ? 1u : 0u);
-          mma_i8(tmem + kDig, sdesc_sw128(smem_u32(Yl) + kt * kSlice + ko), bd, idesc, s ? 1u : 0u);
-        }
-        mma_commit(&H.bar_mma[half]);
-      }
-      if (!mbar_wait(&H.bar_mma[half], phase, err)) H.abort = 1;
-      phase ^= 1;
+    if (tid == 0) {
       tc_fence_after();
-#pragma unroll 1
-      for (int c32 = 0; c32 < kDig; c32 += 32) {
-        u32 zh[32], zl[32];
-        tmem_ld32(tmem + ((u32)((warp & 3) * 32) << 16) + c32, zh);
-        tmem_ld32(tmem + ((u32)((warp & 3) * 32) << 16) + kDig + c32, zl);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          int t0 = ch * kDig + c32 + j;
-          if (t0 >= E) break;
-          // z = 128 Zh + Zl - k Md fits int32: |Zh| <= n 2^14 <= 320 2^14 < 2^23, |Zl| < 2^21, |k Md| < 2^15.
-          // The word's four digits are summed apart from the carry (a tree, independent of the previous
-          // word), so only one 64-bit add per word waits on the carry chain
-          i64 z4[4];
-#pragma unroll
-          for (int u = 0; u < 4; u++)
-            z4[u] = (i64)(128 * (int)zh[j + u] + (int)zl[j + u] - kq32 * TB.md[t0 + u]) * (i64)(1 << (8 * u));
-          const i64 v = carry + ((z4[0] + z4[1]) + (z4[2] + z4[3]));
-          const u32 wv = (u32)v;
-          if (MODE == 0) {
-            if (valid) out[(i64)nw * B + e] = (int32_t)wv;
-            if (wv != 0u) hz = nw, hzv = wv;
-            if (wv != 0xffffffffu) ho = nw, hov = wv;
-            wtop = wv;
-          } else {
-            words[nw] = wv;
+      for (int c = 0; c < nchunk; c++, seq++) {
+        const u32 s = resident ? (u32)c : seq % nslot;
+        if (!mbar_wait(&H.full[s], resident ? 0u : (seq / nslot) & 1u, err)) {
+          H.abort = 1;
+          break;
+        }
+        const u32 tb = smem_u32(slots) + s * cbytes;
+        for (int h = 0; h < 2; h++)
+          for (int ks = 0; ks < ksteps; ks++) {
+            const u32 o = (u32)(h * ktc + (ks >> 2)) * kSlice + (u32)(ks & 3) * 32;
+            mma_i8(tmem + c * kDig, sdesc_sw128(smem_u32(Yh) + o), sdesc_sw128(tb + o), idesc, (h | ks) ? 1u : 0u);
           }
-          nw++;
-          carry = v >> 32;
+        if (!resident) mma_commit(&H.empty[s]);
+      }
+      mma_commit(&H.done);
+    } else if (tid == 32 && !resident) {
+      // refill each slot with the chunk nslot further in the sequence (it wraps over the tiles)
+      for (int c = 0; c < nchunk; c++, seq++) {
+        const u32 s = seq % nslot;
+        if (!mbar_wait(&H.empty[s], (seq / nslot) & 1u, err)) {
+          H.abort = 1;
+          break;
+        }
+        const bool last = tile + gridDim.x >= ntiles;
+        const u32 nx = (u32)c + nslot;        // < 2 nchunk
+        if (nx >= (u32)nchunk && last) continue;
+        mbar_expect_tx(&H.full[s], cbytes);
+        const uint8_t* src = ct + (size_t)(nx % nchunk) * cbytes;
+        for (u32 o = 0; o < cbytes; o += kSlice) bulk_load(slots + s * cbytes + o, src + o, kSlice, &H.full[s]);
+      }
+    }
+    __syncwarp();
+    if (!mbar_wait(&H.done, phase, err)) H.abort = 1;
+    phase ^= 1;
+    tc_fence_after();
+    const int ncol = 4 * (W + 1);
+    u32 za[32], zb[32];
+    auto words8 = [&](int c0, const u32 (&z)[32]) {  // digit columns c0 .. c0 + 31
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const int wd = c0 / 4 + j - 1;
+        if (wd >= W) break;
+        u64 v = digit_word<WIDE>(z + 4 * j);
+        if (j == 0 && wd < 0) {
+          kq = (u32)((v + (1u << 28)) >> 29);
+          continue;
+        }
+        v += (u64)kq * NM[wd];
+        v += carry;
+        const u32 wv = (u32)v;
+        carry = (u32)(v >> 32);
+        if (MODE == 0) {
+          if (valid) out[(i64)wd * B + e] = (int32_t)wv;
+          if (wv != 0u) hz = wd, hzv = wv;
+          if (wv != 0xffffffffu) ho = wd, hov = wv;
+          wtop = wv;
+        } else {
+          col[wd * kThreads] = wv;
         }
       }
-      tc_fence_before();
-      __syncthreads();
+    };
+    tmem_ld32(tmem + lane0, za);
+    for (int c0 = 0; c0 < ncol; c0 += 64) {          // the next 32 columns are read while these are carried
+      tmem_ld_wait();
+      if (c0 + 32 < ncol) tmem_ld32(tmem + lane0 + c0 + 32, zb);
+      words8(c0, za);
+      tmem_ld_wait();
+      if (c0 + 32 >= ncol) break;
+      if (c0 + 64 < ncol) tmem_ld32(tmem + lane0 + c0 + 64, za);
+      words8(c0 + 32, zb);
     }
+    tc_fence_before();
 
     // ---- outputs
     if (valid) {
@@ -205,55 +242,66 @@ __global__ void __launch_bounds__(kThreads * TPC)
         const u32 x = ng ? ~hov : hzv;
         out2[e] = k < 0 ? 0 : 32 * (i64)k + 32 - __clz(x);
       } else {
-        bool ng = words[W - 1] >> 31;
-        if (ng) neg_words(words, W);
-        int bl = bitlen_mag(words, W);
-        if (!bl) {
-          for (int k = 0; k < L; k++) out[(i64)k * B + e] = 0;
-          out2[e] = SDPV_EZ;
-        } else {
-          u32 rr[160];
-          int s = bl - (32 * L - 2);
-          mag_shift(words, W, s, rr, L);
-          if (ng) neg_words(rr, L);
-          for (int k = 0; k < L; k++) out[(i64)k * B + e] = (int32_t)rr[k];
-          out2[e] = rowexp[r] + colexp[(r / rows_per_block) * N + j0 + jj] + s;
-        }
+        col_mpf_norm(col, W, rowexp[r] + colexp[(r / rows_per_block) * N + j0 + jj], L, out + e, B, out2 + e);
       }
     }
+    tile += gridDim.x;
+    if (tile >= ntiles) break;
+    e = tile * 128 + tid;
+    valid = e < B;
+    r = valid ? e / w : 0;
+    jj = valid ? e - r * w : 0;
+    ap = acc + r * N + j0 + jj;
+    load(0, va);
+    __syncthreads();                                   // everyone is done with the columns over Y and with TMEM
+    if (H.abort) break;
   }
   __syncthreads();
-  if (warp == 0) tmem_dealloc(H.tmem_slot, 2 * kDig * TPC);
+  if (H.abort && tid == 0) mbar_wait(&H.done, phase, err);   // a wait gave up: let committed products drain (bounded)
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, tcols);
 }
 
-template <int MODE, int TPC>
+template <int MODE, bool WIDE>
 int launch_crt_t(const sdpv_ctx* c, const int16_t* acc, i64 ldg, i64 N, i64 j0, i64 w, i64 rows, i64 rpb,
                  const int64_t* rowexp, const int64_t* colexp, int L, int32_t* out, int64_t* out2, cudaStream_t st,
-                 const int32_t* pred, size_t smem) {
+                 const int32_t* pred) {
   const CtxDev& d = c->d;
+  const int nchunk = d.Epad / kDig;
+  const size_t chunk = (size_t)2 * d.ktc * kSlice, fixed = 1024 + kHead + chunk;      // Y is as large as a chunk
+  int nslot = (int)((227 * 1024 - fixed) / chunk);      // 2 slots of 64 KB for ktc = 2
+  if (nslot > nchunk) nslot = nchunk;
+  u32 tcols = 128;
+  while ((int)tcols < kDig * nchunk) tcols *= 2;
+  // CTAs per SM: what shared memory and TMEM hold, at most the tuned count (and no more may become resident
+  // than TMEM serves)
+  size_t smem = fixed + nslot * chunk;
+  const int by_tmem = 512 / (int)tcols;
+  int per_sm = (int)((228 * 1024) / (smem + 1024));
+  if (per_sm > by_tmem) {
+    per_sm = by_tmem;
+    smem = (228 * 1024) / (by_tmem + 1);
+  }
+  const int tuned = sdpv::tune(SDPV_TUNE_CRT_CTAS);
+  if (per_sm > tuned) per_sm = tuned;
+  if (per_sm < 1) per_sm = 1;
   static bool attr_set[64] = {};
-  static size_t attr_val[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (!attr_set[dev & 63] || attr_val[dev & 63] < smem) {
-    cudaError_t e = cudaFuncSetAttribute(crt_kernel<MODE, TPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (!attr_set[dev & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(crt_kernel<MODE, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         227 * 1024);
     if (e != cudaSuccess) return set_cuda_error(e);
     attr_set[dev & 63] = true;
-    attr_val[dev & 63] = smem;
   }
-  i64 B = rows * w;
-  i64 ntiles = (B + 127) / 128, nunits = (ntiles + TPC - 1) / TPC;
+  const i64 ntiles = (rows * w + 127) / 128;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // CTAs per SM: the tuned count for one-tile CTAs; two-tile CTAs as many as shared memory holds (at most 2)
-  i64 per_sm = TPC == 1 ? (i64)sdpv::tune(SDPV_TUNE_CRT_CTAS) : (i64)((228 * 1024) / (smem + 1024));
-  if (per_sm < 1) per_sm = 1;
-  if (TPC == 2 && per_sm > 2) per_sm = 2;
-  i64 gx = per_sm * sms;
-  if (gx > nunits) gx = nunits;
-  crt_kernel<MODE, TPC><<<(unsigned)gx, kThreads * TPC, smem, st>>>(
-      acc, ldg, N, j0, w, rows, rpb, rowexp, colexp, L, d.n, d.E, d.W, d.ktc, d.Epad, d.mods, d.minv, d.inv, d.md,
-      d.ct, out, out2, pred, device_error_word());
+  i64 gx = (i64)per_sm * sms;
+  if (gx > ntiles) gx = ntiles;
+  crt_kernel<MODE, WIDE><<<(unsigned)gx, kThreads, smem, st>>>(
+      acc, ldg, N, j0, w, rows, rpb, rowexp, colexp, L, d.n, d.W, d.ktc, nchunk, nslot, tcols, d.crtmod, d.negm, d.ct,
+      out, out2, pred, device_error_word());
   return launch_status();
 }
 
@@ -262,14 +310,11 @@ int launch_crt(const sdpv_ctx* c, const int16_t* acc, i64 ldg, i64 N, i64 j0, i6
                const int64_t* rowexp, const int64_t* colexp, int L, int32_t* out, int64_t* out2, cudaStream_t st,
                const int32_t* pred = nullptr) {
   const CtxDev& d = c->d;
-  if (d.n > kNmax || d.E > kEmax) return SDPV_EINVAL;
-  const size_t tables = (size_t)(d.Epad / 128) * d.ktc * kSlice, tile = (size_t)2 * d.ktc * kSlice;
-  const size_t smem1 = 1024 + 8192 + tile + tables, smem2 = 1024 + 8192 + 2 * tile + tables;
-  // two tiles per CTA when two such CTAs fit an SM (shared memory) and there are tiles for them
-  if (smem2 <= 112 * 1024 && rows * w > 128 * 148)
-    return launch_crt_t<MODE, 2>(c, acc, ldg, N, j0, w, rows, rpb, rowexp, colexp, L, out, out2, st, pred, smem2);
-  if (smem1 > 227 * 1024) return SDPV_EINVAL;
-  return launch_crt_t<MODE, 1>(c, acc, ldg, N, j0, w, rows, rpb, rowexp, colexp, L, out, out2, st, pred, smem1);
+  // at most 256 moduli (L <= 59); there 4 + E <= 512 and a word column fits the 64 ktc words of an entry in Y
+  if (d.n > kNmax || d.Epad > kSlots * kDig || d.W > kWmax || d.W > 64 * d.ktc) return SDPV_EINVAL;
+  if (d.n > 168)
+    return launch_crt_t<MODE, true>(c, acc, ldg, N, j0, w, rows, rpb, rowexp, colexp, L, out, out2, st, pred);
+  return launch_crt_t<MODE, false>(c, acc, ldg, N, j0, w, rows, rpb, rowexp, colexp, L, out, out2, st, pred);
 }
 
 }  // namespace

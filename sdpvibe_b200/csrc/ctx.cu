@@ -43,19 +43,6 @@ struct Big {  // little-endian 32-bit words
       if (w[i]) return 32 * (int)i + 32 - __builtin_clz(w[i]);
     return 0;
   }
-  // Signed base-256 digits in [-128, 128), `count` of them (x must fit).
-  std::vector<int> sdigits256(int count) const {
-    std::vector<int> out(count);
-    int carry = 0;
-    for (int t = 0; t < count; t++) {
-      int b = (t / 4 < (int)w.size()) ? (int)((w[t / 4] >> (8 * (t % 4))) & 255u) : 0;
-      int v = b + carry;
-      int r = ((v + 128) & 255) - 128;
-      out[t] = r;
-      carry = (v - r) / 256;
-    }
-    return out;
-  }
 };
 
 std::vector<int> primes_desc(int hi, int lo) {  // primes p with lo < p <= hi, descending
@@ -126,7 +113,7 @@ extern "C" int sdpv_ctx_create_g(int L, int G, sdpv_ctx** out) {
   d.kt = (NB + 2 + 127) / 128;   // limb bytes + a constant byte + a sign byte
   d.ktc = (n + 127) / 128;
   d.npad16 = (n + 31) / 32 * 32;
-  d.Epad = (E + 127) / 128 * 128;
+  d.Epad = (4 + E + 127) / 128 * 128;
 
   std::vector<int32_t> vm(n), vc14(n), vc1(n), vc1m2(n), vinv(n);
   std::vector<float> vminv(n);
@@ -181,22 +168,37 @@ extern "C" int sdpv_ctx_create_g(int L, int G, sdpv_ctx** out) {
     Mi.divmod_small((u32)m);
     vinv[g] = (int32_t)invmod(Mi.mod_small((u32)m), m);
   }
-  // CRT digits: Ct[t][i] = signed base-256 digit t of M/m_i; B operand rows = digits, K = moduli.
+  // CRT digit table (crt.cu): rows = output digits, K = the two unsigned digits of y_i (y = 128 yh + yl).  Row
+  // 4 + t holds digit t (base 256, unsigned) of 128 M/m_i against yh_i and of M/m_i against yl_i; rows 0 .. 2
+  // the digits of 128 w_i and w_i, w_i = round(2^29 / m_i): the fixed-point sum of y_i / m_i that gives k.
   int nchunks = d.Epad / 128;
-  std::vector<uint8_t> ct((size_t)nchunks * d.ktc * 128 * 128, 0);
+  std::vector<uint8_t> ct((size_t)nchunks * 2 * d.ktc * 128 * 128, 0);
+  std::vector<sdpv::CrtMod> vcm((size_t)d.ktc * 128, sdpv::CrtMod{0, 0, 0.f, 0});
   for (int i = 0; i < n; i++) {
+    const u32 m = (u32)mods[i];
+    vcm[i] = {(int32_t)m, vinv[i], (float)((double)vinv[i] / (double)m), (int32_t)(0x4B400000u * m)};
     Big Mi = M;
-    Mi.divmod_small((u32)mods[i]);
-    std::vector<int> dg = Mi.sdigits256(E);
-    for (int t = 0; t < E; t++) {
-      int chunk = t / 128, row = t % 128, kt = i / 128, col = i % 128;
-      size_t base = ((size_t)chunk * d.ktc + kt) * 128 * 128;
-      ct[base + sw128_off(row, col / 16) + (col % 16)] = (uint8_t)(int8_t)dg[t];
+    Mi.divmod_small(m);
+    Big wi;
+    wi.w = {(u32)(((1u << 29) + m / 2) / m)};
+    for (int h = 0; h < 2; h++) {                      // 0: against yl, 1: against yh (times 128)
+      if (h) Mi.mul_small(128), wi.mul_small(128);
+      auto put = [&](int row, const Big& v, int t) {
+        const u32 b = (t / 4 < (int)v.w.size()) ? (v.w[t / 4] >> (8 * (t % 4))) & 255u : 0u;
+        const size_t slice = ((size_t)(row / 128) * 2 * d.ktc + (h ? 0 : d.ktc) + i / 128) * 128 * 128;
+        ct[slice + sw128_off(row % 128, (i % 128) / 16) + (i % 16)] = (uint8_t)b;
+      };
+      for (int t = 0; t < 4; t++) put(t, wi, t);
+      for (int t = 0; t < E; t++) put(4 + t, Mi, t);
     }
   }
-  std::vector<int> mdg = M.sdigits256(E);
-  std::vector<int32_t> vmd(d.Epad, 0);
-  for (int t = 0; t < E; t++) vmd[t] = mdg[t];
+  std::vector<u32> vnm(E / 4);                          // words of 2^(8E) - M
+  u64 cy = 1;
+  for (int k = 0; k < E / 4; k++) {
+    cy += (u32)~(k < (int)M.w.size() ? M.w[k] : 0u);
+    vnm[k] = (u32)cy;
+    cy >>= 32;
+  }
 
   int st = SDPV_OK;
   if (!st) st = upload(&d.mods, vm);
@@ -204,8 +206,8 @@ extern "C" int sdpv_ctx_create_g(int L, int G, sdpv_ctx** out) {
   if (!st) st = upload(&d.c14, vc14);
   if (!st) st = upload(&d.c1, vc1);
   if (!st) st = upload(&d.c1m2, vc1m2);
-  if (!st) st = upload(&d.inv, vinv);
-  if (!st) st = upload(&d.md, vmd);
+  if (!st) st = upload(&d.crtmod, vcm);
+  if (!st) st = upload(&d.negm, vnm);
   if (!st) st = upload(&d.tab, tab);
   if (!st) st = upload(&d.tabu, tabu);
   if (!st) st = upload(&d.ct, ct);
@@ -222,7 +224,7 @@ extern "C" int sdpv_ctx_create_g(int L, int G, sdpv_ctx** out) {
 extern "C" int sdpv_ctx_destroy(sdpv_ctx* c) {
   if (!c) return SDPV_OK;
   sdpv::CtxDev& d = c->d;
-  void* ptrs[] = {d.mods, d.minv, d.c14, d.c1, d.c1m2, d.inv, d.md, d.tab, d.tabu, d.ct};
+  void* ptrs[] = {d.mods, d.minv, d.c14, d.c1, d.c1m2, d.crtmod, d.negm, d.tab, d.tabu, d.ct};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   delete[] c->mods_host;

@@ -145,7 +145,7 @@ __device__ __forceinline__ void col_magnitude(u32* c, int n, bool neg) {
 // Any product (operands not normalised, or the short product's guard word undecided): the whole product
 // twice, first for its bit length, then shifted, rounded and written as its words appear; nothing is stored.
 // Rare, so it is kept out of line.
-__device__ __noinline__ int col_mul_general(const u32* a, const u32* b, int nb, int L, bool neg, int32_t* out,
+static __device__ __noinline__ int col_mul_general(const u32* a, const u32* b, int nb, int L, bool neg, int32_t* out,
                                             i64 plane) {
   int top = 0;
   col_product(a, b, nb, 0, [&](int kb, const u32 (&w)[4]) {
