@@ -156,6 +156,15 @@ int sdpv_align(const int32_t* m, const int64_t* e, int L, int64_t nb, int64_t R,
  * with bulk tensor copies.  No reference counterpart. */
 int sdpv_align_t(const int32_t* m, const int64_t* e, int L, int64_t nb, int64_t R, int64_t C, const int64_t* target,
                  int per_col, int Lout, int64_t Rld, int32_t* out, void* stream);
+/* The set-up of C = op(A) op(B) (nb blocks, op(A) (M, K), op(B) (K, N); stored A is (nb, K, M) when transA,
+ * stored B (nb, N, K) when transB): the rows of op(A) and the columns of op(B) aligned to their own exponents
+ * max(top) - (32L - 2) (0 for all-zero vectors), as sdpv_top_max + sdpv_align do per operand, into one stacked
+ * buffer X (L, nb M + nb N, ld): the nb M rows of op(A), then the nb N columns of op(B), K entries each (entries
+ * K .. ld - 1 untouched).  Ea (nb, M) and Eb (nb, ldE >= N) receive the exponents.  L <= 64, sizes >= 1.
+ * Replaces both mpf._align_rows of mpf.gemm (sdpvibe/mpf.py:390-398, 410-420). */
+int sdpv_gemm_operands(const int32_t* Am, const int64_t* Ae, const int32_t* Bm, const int64_t* Be, int L, int64_t nb,
+                       int64_t M, int64_t K, int64_t N, int transA, int transB, int64_t ld, int32_t* X, int64_t* Ea,
+                       int64_t* Eb, int64_t ldE, void* stream);
 /* The transposed alignment written as operand rows for sdpv_residues_rows: entry (b, r, c) of m becomes row
  * (b C + c) Rp + r of out (nb, C, Rp, rb) uint8, rb = 128 bytes for Lout <= 31, 256 for Lout <= 63: the Lout
  * aligned limbs little endian, then a sign byte (1 when the result is negative) at byte 4 Lout, then zeros;

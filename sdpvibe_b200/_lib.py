@@ -46,6 +46,7 @@ _SIGS = {
     "sdpv_bigfloat_unpack": [_P, _P, _L, _I, _I, _P, _P, _P],
     "sdpv_bigfloat_pack": [_P, _P, _L, _I, _I, _P, _P, _P],
     "sdpv_top_max": [_P, _P, _I, _L, _L, _L, _I, _P, _P],
+    "sdpv_gemm_operands": [_P, _P, _P, _P, _I, _L, _L, _L, _L, _I, _I, _L, _P, _P, _P, _L, _P],
     "sdpv_align": [_P, _P, _I, _L, _L, _L, _P, _I, _I, _I, _P, _P],
     "sdpv_residues": [_P, _P, _L, _L, _L, _L, _I, _I, _P, _P, _L, _P],
     "sdpv_residues_u8": [_P, _P, _L, _L, _L, _L, _I, _I, _P, _P, _L, _P],

@@ -6,9 +6,11 @@
 // (ties toward +infinity), after a transposing copy.  Here:
 //   sdpv_top_max: the reduction in one launch (rows: one warp per row; columns: column strips with a
 //                 64-bit atomic max), reading only the top limbs of normalised data;
-//   sdpv_align:   the rounding shift fused with the transpose: a 16 x 32 tile of entries is staged in
-//                 shared memory with all its limbs (coalesced along columns), then each thread rounds
-//                 its entries and writes the output limb planes coalesced along the new fast axis.
+//   sdpv_align:   the rounding shift fused with the transpose: a tile of entries is staged in shared memory
+//                 with all its limbs (coalesced along columns), then each thread rounds its entries and writes
+//                 the output limb planes coalesced along the new fast axis;
+//   sdpv_gemm_operands: both operands of a product -- reference exponents of all vectors in one launch, both
+//                 alignments in a second one, into one stacked operand buffer.
 #include "common.cuh"
 
 namespace {
@@ -170,16 +172,13 @@ __global__ void align_kernel(const int32_t* __restrict__ m, const i64* __restric
 // apart, which puts the 8 rows x 4 columns that a warp's lanes read at once in distinct banks.
 constexpr int TR = 16, TC = 32;
 constexpr int ATR = 8, ATP = 36;
-__global__ void __launch_bounds__(kThreads) align_t_kernel(const int32_t* __restrict__ m, const i64* __restrict__ e,
-                                                           int L, i64 nb, i64 R, i64 C, const i64* __restrict__ target,
-                                                           int per_col, int Lout, i64 Rld, int32_t* __restrict__ out,
-                                                           unsigned* err) {
-  extern __shared__ u32 sm[];                       // [L][ATR][ATP] limbs, then [ATR][TC + 1] exponents
-  i64* se = reinterpret_cast<i64*>(sm + (size_t)L * ATR * ATP);
-  const i64 n = nb * R * C, no = nb * C * Rld;      // input / output plane sizes
-  const i64 b = blockIdx.z;
-  const i64 nct = (C + TC - 1) / TC;
-  const i64 r0 = (i64)(blockIdx.x / nct) * ATR, c0 = (i64)(blockIdx.x % nct) * TC;
+// One tile (rows r0 .., columns c0 .. of block b); target: block b's exponents per column or row; out: block b's
+// first output row.
+__device__ __forceinline__ void align_tile(u32* sm, const int32_t* __restrict__ m, const i64* __restrict__ e, int L,
+                                           i64 n, i64 b, i64 R, i64 C, i64 r0, i64 c0, const i64* __restrict__ target,
+                                           int per_col, int Lout, int32_t* __restrict__ out, i64 Rld, i64 no,
+                                           unsigned* err) {
+  i64* se = reinterpret_cast<i64*>(sm + (size_t)L * ATR * ATP);   // after [L][ATR][ATP] limbs
   const int tid = threadIdx.x;
   for (int pos = tid; pos < ATR * TC; pos += kThreads) {     // all copies in flight at once
     const int rr = pos / TC, cc = pos % TC;
@@ -204,10 +203,170 @@ __global__ void __launch_bounds__(kThreads) align_t_kernel(const int32_t* __rest
     i64 r = r0 + rr, c = c0 + cc;
     if (r >= R || c >= C) continue;
     i64 ev = se[rr * (TC + 1) + cc];
-    i64 s = (ev == SDPV_EZ) ? (1ll << 30) : target[per_col ? b * C + c : b * R + r] - ev;
+    i64 s = (ev == SDPV_EZ) ? (1ll << 30) : target[per_col ? c : r] - ev;
     const u32* base = sm + rr * ATP + cc;
-    shift_entry32([&](int i) { return base[i * ATR * ATP]; }, L, s, Lout, out + (b * C + c) * Rld + r, no, err);
+    shift_entry32([&](int i) { return base[i * ATR * ATP]; }, L, s, Lout, out + c * Rld + r, no, err);
   }
+}
+
+__global__ void __launch_bounds__(kThreads) align_t_kernel(const int32_t* __restrict__ m, const i64* __restrict__ e,
+                                                           int L, i64 nb, i64 R, i64 C, const i64* __restrict__ target,
+                                                           int per_col, int Lout, i64 Rld, int32_t* __restrict__ out,
+                                                           unsigned* err) {
+  extern __shared__ u32 sm[];
+  const i64 b = blockIdx.z, nct = (C + TC - 1) / TC;
+  align_tile(sm, m, e, L, nb * R * C, b, R, C, (i64)(blockIdx.x / nct) * ATR, (i64)(blockIdx.x % nct) * TC,
+             target + b * (per_col ? C : R), per_col, Lout, out + b * C * Rld, Rld, nb * C * Rld, err);
+}
+
+// ---------------------------------------------------------------- both operands of a product
+// Two launches (tops with the exponent rule, alignments) in place of two reductions, two fills, eight elementwise
+// launches for the rule and two alignments; the stacked output then needs one decomposition for both sides.  A
+// 17 x 12 x 20 product at L = 10 takes 49 us (5 launches) instead of 193 (17), 256 x 256 x 256 at L = 24 93 instead
+// of 193: those are launch-bound.  kTopRows = 512 strided rows per CTA: up to there one CTA sees a whole strip and
+// writes exponents directly; beyond, the strip is split (7380 rows x 1000: 24 us) at the price of a fill and a
+// conversion launch.
+// One operand, stored (nb, R, C).  strided = 0: its vectors are the rows (vector v = b R + r, contiguous);
+// strided = 1: the columns (v = b C + c, stride C).  Vector v's exponent is E[(v / per) ldE + v % per], per =
+// vectors per block, and its aligned limbs are row `row0 + v` of the stacked buffer.
+struct OpSide {
+  const int32_t* m;
+  const i64* e;
+  i64 nb, R, C;
+  int strided;
+  i64 *E, ldE, row0;
+  i64 blocks;          // CTAs of the current launch
+  int split;           // strided: CTAs per 32-column strip (E holds raw tops if > 1)
+  __host__ __device__ i64 per() const { return strided ? C : R; }
+};
+
+__device__ __forceinline__ i64 exponent_of(i64 top, int L) {       // sdpvibe/mpf.py:394-395
+  const i64 E = top - (32 * L - 2);
+  return E < SDPV_EZ / 2 ? 0 : E;
+}
+
+constexpr int kTopRows = 512;          // strided rows per CTA
+constexpr int kWarpVec = 512;          // longest contiguous vector of one warp; longer ones take a CTA
+
+__device__ __forceinline__ i64 top_of(i64 ev, int32_t tw, const OpSide& S, i64 plane, i64 idx, int L) {
+  if (ev == SDPV_EZ) return SDPV_EZ;
+  const u32 x = (u32)tw ^ (tw < 0 ? 0xffffffffu : 0u);
+  if (x) return ev + 32 * (i64)(L - 1) + 32 - __clz(x);            // normalised data: the top limb decides
+  return entry_top(S.m, plane, idx, L, ev);
+}
+
+// Reference exponents of both operands.  All loads of a thread's 16 entries are issued before any is used.
+__global__ void __launch_bounds__(kThreads) gemm_tops_kernel(OpSide A, OpSide B, int L) {
+  __shared__ i64 red[8][32];
+  const bool second = blockIdx.x >= A.blocks;
+  const OpSide& S = second ? B : A;
+  i64 blk = blockIdx.x - (second ? A.blocks : 0);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const i64 plane = S.nb * S.R * S.C;
+  const int32_t* mt = S.m + (i64)(L - 1) * plane;
+  i64 best = SDPV_EZ;
+  if (!S.strided) {
+    const i64 nvec = S.nb * S.R;
+    const bool wide = S.C > kWarpVec;                              // one vector per CTA, else one per warp
+    const i64 v = wide ? blk : blk * 8 + warp;
+    const int t0 = wide ? threadIdx.x : lane, step = wide ? kThreads : 32;
+    if (v < nvec)
+      for (i64 c0 = t0; c0 < S.C; c0 += 16 * step) {
+        i64 ev[16];
+        int32_t tw[16];
+#pragma unroll
+        for (int t = 0; t < 16; t++) {
+          const i64 c = c0 + t * step;
+          ev[t] = c < S.C ? S.e[v * S.C + c] : SDPV_EZ;
+          tw[t] = c < S.C ? mt[v * S.C + c] : 0;
+        }
+#pragma unroll
+        for (int t = 0; t < 16; t++) {
+          const i64 top = top_of(ev[t], tw[t], S, plane, v * S.C + c0 + t * step, L);
+          best = top > best ? top : best;
+        }
+      }
+    for (int o = 16; o > 0; o >>= 1) {
+      const i64 x = __shfl_xor_sync(0xffffffffu, best, o);
+      best = x > best ? x : best;
+    }
+    if (wide) {
+      if (lane == 0) red[warp][0] = best;
+      __syncthreads();
+      if (threadIdx.x == 0)
+        for (int w = 1; w < 8; w++) best = red[w][0] > best ? red[w][0] : best;
+    }
+    if (v < nvec && (wide ? threadIdx.x == 0 : lane == 0)) S.E[(v / S.R) * S.ldE + v % S.R] = exponent_of(best, L);
+    return;
+  }
+  const i64 part = blk % S.split;
+  blk /= S.split;
+  const i64 strips = (S.C + 31) / 32, b = blk / strips, c = (blk - b * strips) * 32 + lane;
+  const i64 r1 = (part + 1) * kTopRows < S.R ? (part + 1) * kTopRows : S.R;
+  if (c < S.C)
+    for (i64 r0 = part * kTopRows + warp * 16; r0 < r1; r0 += 128) {
+      i64 ev[16];
+      int32_t tw[16];
+#pragma unroll
+      for (int t = 0; t < 16; t++) {
+        const i64 idx = (b * S.R + r0 + t) * S.C + c;
+        ev[t] = r0 + t < r1 ? S.e[idx] : SDPV_EZ;
+        tw[t] = r0 + t < r1 ? mt[idx] : 0;
+      }
+#pragma unroll
+      for (int t = 0; t < 16; t++) {
+        const i64 top = top_of(ev[t], tw[t], S, plane, (b * S.R + r0 + t) * S.C + c, L);
+        best = top > best ? top : best;
+      }
+    }
+  red[warp][lane] = best;
+  __syncthreads();
+  if (warp == 0 && c < S.C) {
+#pragma unroll
+    for (int w = 1; w < 8; w++) best = red[w][lane] > best ? red[w][lane] : best;
+    i64* out = S.E + b * S.ldE + c;
+    if (S.split > 1) atomicMax((long long*)out, (long long)best);
+    else *out = exponent_of(best, L);
+  }
+}
+
+// Raw tops of a split side -> exponents.
+__global__ void gemm_exps_kernel(OpSide S, int L) {
+  const i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= S.nb * S.per()) return;
+  i64* p = S.E + (v / S.per()) * S.ldE + v % S.per();
+  *p = exponent_of(*p, L);
+}
+
+// Both alignments: rows are staged entry by entry (one thread per entry, its limbs in a shared-memory column,
+// all copies in flight at once), columns through the transposing tiles of align_t_kernel.  Output row length ld
+// (entries past the vector's length unset), plane stride (rows of both) x ld.
+__global__ void __launch_bounds__(kThreads) gemm_align_kernel(OpSide A, OpSide B, int L, i64 ld, i64 plane_out,
+                                                              int32_t* __restrict__ X, unsigned* err) {
+  extern __shared__ u32 sm[];
+  const bool second = blockIdx.x >= A.blocks;
+  const OpSide& S = second ? B : A;
+  const i64 blk = blockIdx.x - (second ? A.blocks : 0);
+  const int tid = threadIdx.x;
+  const i64 n = S.nb * S.R * S.C;
+  if (!S.strided) {
+    const i64 idx = blk * kThreads + tid;
+    if (idx >= n) return;
+    u32* col = sm + tid;
+    const int32_t* src = S.m + idx;
+#pragma unroll 8
+    for (int l = 0; l < L; l++, src += n) cp_async4(col + l * kThreads, src, 4u);
+    cp_async_commit();
+    const i64 v = idx / S.C, k = idx - v * S.C, ev = S.e[idx];
+    const i64 s = (ev == SDPV_EZ) ? (1ll << 30) : S.E[(v / S.R) * S.ldE + v % S.R] - ev;
+    cp_async_wait<0>();
+    shift_entry32([&](int i) { return col[i * kThreads]; }, L, s, L, X + (S.row0 + v) * ld + k, plane_out, err);
+    return;
+  }
+  const i64 nct = (S.C + TC - 1) / TC, nrt = (S.R + ATR - 1) / ATR;
+  const i64 b = blk / (nct * nrt), t2 = blk - b * nct * nrt;
+  align_tile(sm, S.m, S.e, L, n, b, S.R, S.C, (t2 / nct) * ATR, (t2 % nct) * TC, S.E + b * S.ldE, 1, L,
+             X + (S.row0 + b * S.C) * ld, ld, plane_out, err);
 }
 
 // shift_entry / shift_entry32 with the Lout output words in registers (o[k], k < Lout < RW; loops unrolled to
@@ -437,5 +596,60 @@ extern "C" int sdpv_align_t(const int32_t* m, const int64_t* e, int L, int64_t n
     dim3 grid((unsigned)tiles, 1, (unsigned)nb);
     align_t_kernel<<<grid, kThreads, smem, st>>>(m, e, L, nb, R, C, target, per_col, Lout, Rld, out, err);
   }
+  return sdpv::launch_status();
+}
+
+// Both operands of C = op(A) op(B), aligned and stacked: X (L, nb M + nb N, ld) holds the nb M rows of op(A),
+// then the nb N columns of op(B), K entries each; Ea (nb M) and Eb (nb rows of ldE) their exponents.
+extern "C" int sdpv_gemm_operands(const int32_t* Am, const int64_t* Ae, const int32_t* Bm, const int64_t* Be, int L,
+                                  int64_t nb, int64_t M, int64_t K, int64_t N, int transA, int transB, int64_t ld,
+                                  int32_t* X, int64_t* Ea, int64_t* Eb, int64_t ldE, void* stream) {
+  if (L < 1 || L > 64 || nb < 1 || M < 1 || K < 1 || N < 1 || ld < K || ldE < N || nb > 65535) return SDPV_EINVAL;
+  cudaStream_t st = sdpv::as_stream(stream);
+  // a single column is contiguous: it is read as a row
+  OpSide A{Am, Ae, nb, transA ? K : M, transA ? M : K, transA && M > 1, Ea, M, 0, 0, 1};
+  OpSide B{Bm, Be, nb, transB ? N : K, transB ? K : N, !transB && N > 1, Eb, ldE, nb * M, 0, 1};
+  if (transA && M == 1) A.R = 1, A.C = K;
+  if (!transB && N == 1) B.R = 1, B.C = K;
+  bool raw = false;
+  for (OpSide* S : {&A, &B}) {
+    if (S->strided) {
+      S->split = (int)((S->R + kTopRows - 1) / kTopRows);
+      S->blocks = S->nb * ((S->C + 31) / 32) * S->split;
+      raw = raw || S->split > 1;
+    } else {
+      S->blocks = S->C > kWarpVec ? S->nb * S->R : (S->nb * S->R + 7) / 8;
+    }
+  }
+  if (A.blocks + B.blocks > 0x7fffffff) return SDPV_EINVAL;
+  if (raw) {
+    // tops of split columns meet by atomic maximum: start below every top (0x80 bytes are below EZ)
+    for (OpSide* S : {&A, &B})
+      if (S->split > 1) {
+        const size_t count = (size_t)((S->nb - 1) * S->ldE + S->per());
+        cudaError_t ce = cudaMemsetAsync(S->E, 0x80, count * 8, st);
+        if (ce != cudaSuccess) return sdpv::set_cuda_error(ce);
+      }
+  }
+  gemm_tops_kernel<<<(unsigned)(A.blocks + B.blocks), kThreads, 0, st>>>(A, B, L);
+  for (OpSide* S : {&A, &B})
+    if (S->split > 1) gemm_exps_kernel<<<blocks(S->nb * S->per()), kThreads, 0, st>>>(*S, L);
+  for (OpSide* S : {&A, &B})
+    S->blocks = S->strided ? S->nb * ((S->C + TC - 1) / TC) * ((S->R + ATR - 1) / ATR)
+                           : (S->nb * S->R * S->C + kThreads - 1) / kThreads;
+  if (A.blocks + B.blocks > 0x7fffffff) return SDPV_EINVAL;
+  const size_t tile = (size_t)L * ATR * ATP * 4 + ATR * (TC + 1) * 8, cols = (size_t)L * kThreads * 4;
+  const size_t smem = A.strided || B.strided ? tile : cols;         // a transposing tile is the larger
+  static bool attr[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!attr[dev & 63]) {
+    cudaError_t ce = cudaFuncSetAttribute(gemm_align_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          64 * ATR * ATP * 4 + ATR * (TC + 1) * 8);
+    if (ce != cudaSuccess) return sdpv::set_cuda_error(ce);
+    attr[dev & 63] = true;
+  }
+  gemm_align_kernel<<<(unsigned)(A.blocks + B.blocks), kThreads, smem, st>>>(A, B, L, ld, nb * (M + N) * ld, X,
+                                                                            sdpv::device_error_word());
   return sdpv::launch_status();
 }

@@ -16,7 +16,7 @@ import torch
 
 from . import _lib, graphs
 from .limbops import shift_round, bitlen_words
-from .mpmat import lib_ctx, KC_MAX, RES_BUDGET
+from .mpmat import lib_ctx, stacked_product
 from .rns import dev
 
 EZ = -(1 << 40)                                      # exponent of zero (sdpvibe/mpf.py:21)
@@ -381,31 +381,37 @@ def _align_rows(A):
 def gemm(A, B, transA=False, transB=False):
     """C = op(A) op(B) (2-d, or batched 3-d (nb, ., .)); exact products, every entry rounded once
     (operands aligned per row of op(A) / column of op(B)) (sdpvibe/mpf.py:401-452)."""
-    if A.e.dim() == 2:
-        A1 = MPF(A.m[:, None], A.e[None])
-        B1 = MPF(B.m[:, None], B.e[None])
-        C = gemm(A1, B1, transA, transB)
-        return MPF(C.m[:, 0], C.e[0])
-    # op(A) rows and op(B) columns aligned to their own exponents; the transposes are fused into the
-    # alignment kernel (stored A is (nb, K, M) when transA; stored B is (nb, K, N) unless transB)
-    nb = A.shape[0]
-    M = A.shape[2] if transA else A.shape[1]
-    K = A.shape[1] if transA else A.shape[2]
-    N = B.shape[1] if transB else B.shape[2]
-    K2 = B.shape[2] if transB else B.shape[1]
-    assert K == K2 and B.shape[0] == nb, (A.shape, B.shape)
+    sa, sb = A.e.shape, B.e.shape
+    assert len(sa) == len(sb), (A.shape, B.shape)
+    nb = sa[0] if len(sa) == 3 else 1
+    M, K = (sa[-1], sa[-2]) if transA else (sa[-2], sa[-1])
+    N, K2 = (sb[-2], sb[-1]) if transB else (sb[-1], sb[-2])
+    assert K == K2 and (len(sb) == 2 or sb[0] == nb), (A.shape, B.shape)
     L = A.L
-    rA = _row_exponents(top_max(A, over_rows=transA), L)            # (nb, M)
-    Am = aligned(A, rA, per_col=transA, transpose=transA)          # (L, nb, M, K)
-    cB = _row_exponents(top_max(B, over_rows=not transB), L)        # (nb, N)
-    Bm = aligned(B, cB, per_col=not transB, transpose=not transB)  # (L, nb, N, K)
+    assert B.L == L, (A.L, B.L)
+    shape = (nb, M, N) if len(sa) == 3 else (M, N)
+    if not (nb and M and N and K):
+        return zeros(shape, L)                                      # no entries, or empty sums
+    # op(A) rows and op(B) columns aligned to their own exponents, the transposes fused into the alignment, both
+    # stacked in one operand buffer (rows padded to 16 bytes for the decomposition's bulk copies)
+    ld = (K + 3) & ~3
+    ldc = N if N <= 64 else (N + 7) & ~7                            # 16-byte rows for the GEMM's full tiles
+    X = torch.empty((L, nb * (M + N), ld), dtype=torch.int32, device=dev)
+    E = torch.empty((nb * (M + ldc),), dtype=torch.int64, device=dev)
+    Am, Ae, Bm, Be = A.m.contiguous(), A.e.contiguous(), B.m.contiguous(), B.e.contiguous()
+    ea = E.data_ptr()
+    eb = ea + 8 * nb * M
+    st = _lib.stream()
+    _lib.call("sdpv_gemm_operands", _lib.ptr(Am), _lib.ptr(Ae), _lib.ptr(Bm), _lib.ptr(Be), L, nb, M, K, N,
+              int(transA), int(transB), ld, X.data_ptr(), ea, eb, ldc, st)
     R = lib_ctx(L)
-    acc = (torch.empty if K else torch.zeros)((R.n, nb * M, N), dtype=torch.int16, device=dev)
-    if K:
-        from .mpmat import residue_product
-        residue_product(R, Am.view(L, nb * M, K), Bm.view(L, nb * N, K), acc, nb=nb, fresh=True)
-    Om, Oe = R.crt_norm(acc, N, 0, N, nb * M, rA.reshape(-1), cB, L, rows_per_block=M)
-    return MPF(Om.view(L, nb, M, N), Oe.view(nb, M, N))
+    acc = torch.empty((R.n, nb * M, ldc), dtype=torch.int16, device=dev)
+    stacked_product(R, X, nb, M, N, K, acc, ldc)
+    Om = torch.empty((L, *shape), dtype=torch.int32, device=dev)
+    Oe = torch.empty(shape, dtype=torch.int64, device=dev)
+    _lib.call("sdpv_crt_norm", R.handle, acc.data_ptr(), acc.stride(0), ldc, 0, N, nb * M, M, ea, eb, L, Om.data_ptr(),
+              Oe.data_ptr(), st)
+    return MPF(Om, Oe)
 
 
 def symmetrize(A):

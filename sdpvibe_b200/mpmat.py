@@ -10,7 +10,7 @@ import ctypes
 import torch
 
 from . import _lib
-from .rns import RNS, dev
+from .rns import RNS, dev, plane_stride
 from .limbops import shift_round, add_same, bitlen_words
 
 KC_MAX = 32768            # inner-dimension chunk of one residue GEMM launch (int32 bound of unsigned digits)
@@ -225,6 +225,28 @@ def residue_product(R, Av, Bv, acc, nb=1, syrk=False, fresh=False, kvalid=None):
                 Bh, Bl = R.residues(Bv, k0, kk, g0, G, spread=True, unsigned=True)
                 R.accumulate(Ah, Al, Bh, Bl, acc, g0, nb=nb, fresh=first, unsigned=True)
             del Ah, Al
+
+
+def stacked_product(R, X, nb, M, N, K, acc, ldc):
+    """acc (R.n, nb M, ldc) = residues of the exact products of nb blocks whose operands lie stacked in X (L,
+    nb M + nb N, ld), K of the ld entries of each row used: one decomposition for both sides."""
+    rows, ld = X.shape[1], X.shape[2]
+    per_mod = rows * min(K, KC_MAX) * 2
+    GR = R.n if R.n * per_mod <= RES_BUDGET else max(16, (RES_BUDGET // per_mod) // 16 * 16)
+    st = _lib.stream()
+    for k0 in range(0, K, KC_MAX):
+        kk = min(KC_MAX, K - k0)
+        kp = -(-kk // 16) * 16
+        ps = plane_stride(rows * kp)
+        for g0 in range(0, R.n, GR):
+            G = min(GR, R.n - g0)
+            buf = torch.empty((2 * G * ps,), dtype=torch.uint8, device=dev)
+            hi = buf.data_ptr()
+            lo = hi + G * ps
+            _lib.call("sdpv_residues_u8", R.handle, X.data_ptr(), rows, ld, k0, kk, g0, G, hi, lo, ps, st)
+            ofs = nb * M * kp
+            _lib.call("sdpv_rns_gemm", R.handle, hi, lo, hi + ofs, lo + ofs, ps, ps, acc.data_ptr(), ldc, g0, G, nb, M,
+                      N, kp, 6 if k0 == 0 else 4, st)
 
 
 def residue_product_rows(R, Xr, nI, Rp, K, acc, fresh=False):
