@@ -651,8 +651,12 @@ __global__ void __launch_bounds__(64 + 32 * NW, 1)
       }
     }
     for (i64 item = blockIdx.x; item < nitems && !kNarrowOnly && pack > 1 && !nmode; item += gridDim.x, li++) {
-      // packed small blocks: tile rows are the stacked rows of blocks t*pack .. t*pack + nbt - 1, tile
-      // columns their stacked B rows; only the diagonal sub-blocks are outputs (staged, coalesced)
+      // packed small blocks: tile rows are the stacked rows of blocks t*pack .. t*pack + nbt - 1, tile columns
+      // their stacked B rows; only the diagonal sub-blocks are outputs.  A warp's 32 rows belong to a few
+      // consecutive blocks, so it reads only those blocks' columns (16 at a time, the quarter's two warps
+      // alternating): 47 of 128 on average at M = N = 21 (360 blocks of 21 x 41 x 21 at 116 moduli: 313 -> 160
+      // us per launch against reducing all 128).  Each thread stages its own block's entries; with
+      // ldc = N a tile's outputs are one contiguous run of acc and leave as such.
       const i64 t = item % tiles;
       const int g = (int)(item / tiles);
       const int gg = g0 + gofs + g;
@@ -660,45 +664,53 @@ __global__ void __launch_bounds__(64 + 32 * NW, 1)
       const float minv = S.tminv[g];
       const i64 b0 = t * pack;
       const int nbt = (int)(nb - b0 < pack ? nb - b0 : pack);
-      const int nrow = nbt * (int)M;
+      const int Mi = (int)M, Ni = (int)N, nrow = nbt * Mi;
       const i64 rowbase = (i64)gg * nb * M + b0 * M;               // acc row of tile row 0
-      const int rrow = q * 32 + lane;
-      u32 olds[2][16];
-#pragma unroll
-      for (int c = 0; c < 2; c++)
-#pragma unroll
-        for (int j = 0; j < 16; j++) olds[c][j] = 0;
-      if (!fresh) {
-        epi_sync();
-        for (int r = ew; r < nrow; r += 8) {
-          const int bi = r / (int)M;
-          const int16_t* src = acc + (rowbase + r) * ldc;
-          for (int j = lane; j < N; j += 32) S.stg[r][bi * N + j] = src[j];
-        }
-        epi_sync();
-#pragma unroll
-        for (int c = 0; c < 2; c++)
-#pragma unroll
-          for (int j = 0; j < 16; j++)
-            olds[c][j] = *reinterpret_cast<const u32*>(&S.stg[rrow][64 * ch + 32 * c + 2 * j]);
-      }
+      const int rrow = q * 32 + lane, rlast = min(q * 32 + 31, nrow - 1);
+      const int c0 = (q * 32 / Mi) * Ni, c1 = q * 32 < nrow ? (rlast / Mi + 1) * Ni : c0;
+      const int own = (rrow / Mi) * Ni;                            // this row's first column
+      const int nown = rrow < nrow ? Ni : 0;
+      int16_t* stg = &S.stg[0][0];                                 // [nrow][N], linear
+      const bool small_k = u8ops && KC <= 64;                      // 128 hx < 2^29 needs no reduction of its own
+      const u32 mu = (u32)m, k0 = 0x4B400000u * mu;
+      auto red = [&](int x) -> int {                               // see the narrow items
+        return (int)((u32)x + k0 - (u32)__float_as_int(fmaf((float)x, minv, 12582912.0f)) * mu);
+      };
       const bool ok_me = mbar_wait(&S.acc_full, li & 1, err);
-      const bool fail = epi_sync_or(!ok_me);
+      const bool fail = epi_sync_or(!ok_me);                       // also: the previous tile has left the staging
       if (fail) break;
       tc_fence_after();
-      u32 outp[2][16];
-      epi_compute(tmem, q, ch, lane, m, c14, minv, olds, outp, &S.tmem_empty);
-      epi_sync();
+      for (int cc = c0 + 16 * ch; cc < c1; cc += 32) {
+        u32 hh[16], hx[16], ll[16];
+        const u32 base = tmem + ((u32)(q * 32) << 16) + cc;
+        tmem_ld16(base, hh);
+        tmem_ld16(base + 128, hx);
+        tmem_ld16(base + 256, ll);
+        tmem_ld_wait();
 #pragma unroll
-      for (int c = 0; c < 2; c++)
-#pragma unroll
-        for (int j2 = 0; j2 < 16; j2++)
-          *reinterpret_cast<u32*>(&S.stg[rrow][64 * ch + 32 * c + 2 * j2]) = outp[c][j2];
+        for (int u = 0; u < 16; u++) {
+          const int j = cc + u - own;
+          const bool in = (unsigned)j < (unsigned)nown;
+          const int o = (in && !fresh) ? (int)acc[(rowbase + rrow) * ldc + j] : 0;
+          const int rx = small_k ? (int)hx[u] : red((int)hx[u]);
+          int rr = red(red((int)hh[u]) * c14 + rx * 128 + (int)ll[u] + o);
+          rr += (rr < 0) ? m : 0;
+          if (in) stg[rrow * Ni + j] = (int16_t)rr;
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&S.tmem_empty);                   // accumulators read: the next item's MMAs may start
       epi_sync();
-      for (int r = ew; r < nrow; r += 8) {
-        const int bi = r / (int)M;
-        int16_t* dst = acc + (rowbase + r) * ldc;
-        for (int j = lane; j < N; j += 32) dst[j] = S.stg[r][bi * N + j];
+      const int count = nrow * Ni, et = tid - 64;
+      int16_t* dst = acc + rowbase * ldc;
+      if (ldc != N) {
+        for (int i = et; i < count; i += 256) dst[(i64)(i / Ni) * ldc + i % Ni] = stg[i];
+      } else if (((uintptr_t)dst & 3) == 0) {
+        for (int i = et; i < count / 2; i += 256) reinterpret_cast<u32*>(dst)[i] = reinterpret_cast<const u32*>(stg)[i];
+        if ((count & 1) && et == 0) dst[count - 1] = stg[count - 1];
+      } else {
+        for (int i = et; i < count; i += 256) dst[i] = stg[i];
       }
     }
     for (i64 item = blockIdx.x; item < nitems && !kNarrowOnly && pack <= 1 && !tailTB && !nmode; item += gridDim.x, li++) {
