@@ -14,6 +14,12 @@
 // floor(x / 2^s + 1/2) on two's-complement words (sdpvibe/limbops.py:31-62), the aligned sum of two operands
 // rounded independently to max(ea, eb) + 1 (sdpvibe/batched.py:55-79), per-column output exponents from the
 // maximal bit length (sdpvibe/batched.py:200-231).
+//
+// What bounds them: with few blocks, the latency of an entry's dependent passes.  So an entry's words are copied into
+// a shared-memory column at once (cp.async) and shifted from there, and the entries of a tile or group are spread
+// over several CTAs.  Measured (B200, L = 26, one 274-row matrix, per launch): finish 20 -> 5.9 us, narrow 62 -> 11.6,
+// widen 43 -> 8.3, solve_round 12.8 -> 6.9, merge 6.2 -> 4.0; 600 blocks of 8 ... 160 rows: finish 121 -> 58, narrow
+// 111 -> 84, solve_round 31.5 -> 13.9.
 #include "common.cuh"
 
 namespace {
@@ -27,50 +33,53 @@ struct Arenas {
   i64 plane[kArenas];
 };
 
-// Word i of a two's-complement number of n words read through `at` (sign-extended above, zero below).
-template <class At>
-__device__ __forceinline__ u64 word_ext(At at, int n, i64 i, u64 ext) {
-  if (i < 0) return 0;
-  if (i >= n) return ext;
-  return (u64)at(i);
-}
-
-// Streaming floor(x / 2^s + 1/2): output word k of the rounded value, produced in increasing k.
-struct ShiftStream {
-  i64 q;
-  int r;
-  u64 lo, carry, ext;
+// Two's-complement words of one entry in a shared-memory column of stride T words (word k at c[k T], conflict
+// free; T = the CTA's threads): words below 0 are zero, from n on the sign.
+struct Col {
+  const u32* c;
+  int T, n;
+  u32 ext;
+  __device__ __forceinline__ u32 operator()(int i) const { return i < 0 ? 0u : (i >= n ? ext : c[i * T]); }
 };
-template <class At>
-__device__ __forceinline__ void shr_begin(ShiftStream& st, At at, int n, i64 s) {
-  st.ext = ((u32)at(n - 1) >> 31) ? 0xffffffffull : 0ull;
-  st.q = s >> 5;
-  st.r = (int)(s - 32 * st.q);
-  const i64 sb = s - 1, qb = sb >> 5;
-  const int rb = (int)(sb - 32 * qb);
-  st.carry = sb >= 0 ? ((word_ext(at, n, qb, st.ext) >> rb) & 1ull) : 0ull;
-  st.lo = word_ext(at, n, st.q, st.ext);
+__device__ __forceinline__ Col make_col(const u32* c, int T, int n) {
+  return Col{c, T, n, (c[(n - 1) * T] >> 31) ? 0xffffffffu : 0u};
 }
-template <class At>
-__device__ __forceinline__ u32 shr_next(ShiftStream& st, At at, int n, int k) {
-  const u64 hi = word_ext(at, n, st.q + k + 1, st.ext);
-  const u64 v = ((((hi << 32) | st.lo) >> st.r) & 0xffffffffull) + st.carry;
-  st.lo = hi;
-  st.carry = v >> 32;
-  return (u32)v;
+// Shift amounts past these bounds give the same words: all sign above, all zero below.
+__device__ __forceinline__ int clamp_shift(i64 s, int n, int nout) {
+  const i64 hi = 32 * (i64)(n + 1), lo = -32 * (i64)(nout + 1);
+  return (int)(s > hi ? hi : (s < lo ? lo : s));
 }
-// The whole rounded value into out[0 .. nout).
-template <class At>
-__device__ __forceinline__ void shr_all(At at, int n, i64 s, u32* out, int nout) {
-  ShiftStream st;
-  shr_begin(st, at, n, s);
-  for (int k = 0; k < nout; k++) out[k] = shr_next(st, at, n, k);
+// Streaming floor(x / 2^s + 1/2) of the words w: output word k in ascending order.
+template <class Word>
+struct Shr {
+  Word w;
+  int q, r;
+  u32 lo, carry;
+  __device__ __forceinline__ Shr(Word w_, int s) : w(w_), q(s >> 5), r(s & 31) {
+    carry = s > 0 ? (w((s - 1) >> 5) >> ((s - 1) & 31)) & 1u : 0u;
+    lo = w(q);
+  }
+  __device__ __forceinline__ u32 next(int k) {
+    const u32 hi = w(q + k + 1);
+    const u32 f = __funnelshift_r(lo, hi, r), v = f + carry;
+    carry = v < f ? 1u : 0u;
+    lo = hi;
+    return v;
+  }
+};
+template <class Word>
+__device__ __forceinline__ Shr<Word> make_shr(Word w, int s) { return Shr<Word>(w, s); }
+
+// Words [0, n) of an entry (plane stride `plane`) into a column; every copy in flight at once.
+__device__ __forceinline__ void stage_col(u32* c, int T, const int32_t* src, i64 plane, int n) {
+#pragma unroll 8
+  for (int k = 0; k < n; k++, src += plane, c += T) cp_async4(c, src, 4u);
 }
 
-__device__ __forceinline__ int bitlen_words(const u32* x, int n) {
-  const u32 ext = (x[n - 1] >> 31) ? 0xffffffffu : 0u;
+__device__ __forceinline__ int col_bits(const u32* c, int stride, int n) {
+  const u32 ext = (c[(n - 1) * stride] >> 31) ? 0xffffffffu : 0u;
   for (int k = n - 1; k >= 0; k--) {
-    const u32 v = x[k] ^ ext;
+    const u32 v = c[k * stride] ^ ext;
     if (v) return 32 * k + 32 - __clz(v);
   }
   return 0;
@@ -114,69 +123,102 @@ __global__ void __launch_bounds__(256) grp_copy_kernel(Arenas src, int32_t* __re
 // desc (40 int64): out arena, out base, out ld, base arena (-1: zero), base base, base ld, rows, cols, nsrc (<= 7),
 // then per source: CRT entry base, sign (+1 / -1), shift constant, exponent index (-1: none).  Entry (r, c):
 //   out = base + sum_i sign_i round(W_i[r][c] / 2^s_i) mod 2^(32 L),  s_i = cst_i - xe[idx_i]
-// where W_i[r][c] is the CRT value (W words, planes Ntot apart) at entry crt_base_i + r * w + c.  Four CTAs
-// per descriptor (grid y), each a quarter of the rows: one entry per thread for a 32 x 32 block.
-__global__ void __launch_bounds__(256) grp_finish_fixed_kernel(const int32_t* __restrict__ Wd, int W, i64 Ntot, i64 w,
-                                                               Arenas ar, int L, const i64* __restrict__ xe,
-                                                               const i64* __restrict__ desc) {
+// where W_i[r][c] is the CRT value (W words, planes Ntot apart) at entry crt_base_i + r * w + c.  Eight CTAs per
+// descriptor (grid y), one entry per thread for a 32 x 32 block.  Only the L + 2 words that the rounding reads
+// are staged; the next source is in flight while one is added (the word-by-word loads of a plain loop had set
+// the time: 20 us a launch of few tiles, with 32 of them per factorisation of 9 tile columns).
+constexpr int kFinT = 128;
+__global__ void __launch_bounds__(kFinT) grp_finish_fixed_kernel(const int32_t* __restrict__ Wd, int W, i64 Ntot, i64 w,
+                                                                 Arenas ar, int L, const i64* __restrict__ xe,
+                                                                 const i64* __restrict__ desc) {
+  extern __shared__ u32 cols[];
+  u32* sum = cols + threadIdx.x;                        // L words, then two source columns of L + 2 words
+  u32* buf = sum + L * kFinT;
   const i64* d = desc + 40 * (i64)blockIdx.x;
-  const int oid = (int)d[0], bid = (int)d[3], rows = (int)d[6], cols = (int)d[7];
+  const int oid = (int)d[0], bid = (int)d[3], rows = (int)d[6], ncol = (int)d[7];
   const int ns = (int)d[8] < kMaxSrc ? (int)d[8] : kMaxSrc;
   const i64 obase = d[1], old_ = d[2], bbase = d[4], bld = d[5];
-  const int rpart = (rows + gridDim.y - 1) / gridDim.y, rlo = blockIdx.y * rpart;   // this CTA's rows
-  const int rhi = rlo + rpart < rows ? rlo + rpart : rows;
-  for (int idx = threadIdx.x; idx < (rhi - rlo) * cols; idx += blockDim.x) {
-    const int r = rlo + idx / cols, c = idx % cols;
-    ShiftStream st[kMaxSrc];
-    i64 sg[kMaxSrc];
-    const int32_t* src[kMaxSrc];
-    for (int i = 0; i < ns; i++) {
-      const i64* si = d + 9 + 4 * i;
-      src[i] = Wd + si[0] + (i64)r * w + c;
-      sg[i] = si[1];
-      const i64 s = si[2] - (si[3] >= 0 ? xe[si[3]] : 0);
-      const int32_t* p = src[i];
-      shr_begin(st[i], [&](i64 k) { return (u32)p[k * Ntot]; }, W, s);
-    }
-    const int32_t* bp = bid >= 0 ? ar.p[bid] + bbase + (i64)r * bld + c : nullptr;
+  for (int idx = blockIdx.y * kFinT + threadIdx.x; idx < rows * ncol; idx += gridDim.y * kFinT) {
+    const int r = idx / ncol, c = idx - r * ncol;
+    if (bid >= 0) stage_col(sum, kFinT, ar.p[bid] + bbase + (i64)r * bld + c, ar.plane[bid], L);
+    else
+      for (int k = 0; k < L; k++) sum[k * kFinT] = 0u;
     int32_t* op = ar.p[oid] + obase + (i64)r * old_ + c;
-    i64 carry = 0;
-    for (int k = 0; k < L; k++) {
-      i64 t = carry + (bp ? (i64)(u32)bp[(i64)k * ar.plane[bid]] : 0);
-      for (int i = 0; i < ns; i++) {
-        const int32_t* p = src[i];
-        const u32 v = shr_next(st[i], [&](i64 kk) { return (u32)p[kk * Ntot]; }, W, k);
-        t += sg[i] * (i64)v;
+    const i64 oplane = ar.plane[oid];
+    // words b0 .. of source i: those from the rounding bit's word up to word q + L, and the top (sign) word last
+    auto issue = [&](int i, int& s, int& b0, int& cnt) {
+      const i64* si = d + 9 + 4 * i;
+      s = clamp_shift(si[2] - (si[3] >= 0 ? xe[si[3]] : 0), W, L);
+      const int q = s >> 5;
+      b0 = q - 1 > 0 ? (q - 1 < W - 1 ? q - 1 : W - 1) : 0;
+      const int e = q + L + 1 < W ? (q + L + 1 > b0 ? q + L + 1 : b0) : W;    // [b0, e)
+      cnt = e - b0;
+      const int32_t* src = Wd + si[0] + (i64)r * w + c;
+      u32* dst = buf + (i & 1) * (L + 3) * kFinT;
+      stage_col(dst, kFinT, src + (i64)b0 * Ntot, Ntot, cnt);
+      cp_async4(dst + (L + 2) * kFinT, src + (i64)(W - 1) * Ntot, 4u);
+    };
+    int s0 = 0, b0 = 0, n0 = 0, s1 = 0, b1 = 0, n1 = 0;
+    if (ns > 0) issue(0, s0, b0, n0);
+    cp_async_commit();
+    for (int i = 0; i < ns; i++) {
+      if (i + 1 < ns) issue(i + 1, s1, b1, n1);
+      cp_async_commit();
+      cp_async_wait<1>();
+      const u32* col = buf + (i & 1) * (L + 3) * kFinT;
+      const u32 ext = (col[(L + 2) * kFinT] >> 31) ? 0xffffffffu : 0u;
+      auto st = make_shr([&](int j) { return j < 0 ? 0u : (j >= W ? ext : col[(j - b0) * kFinT]); }, s0);
+      const bool last = i + 1 == ns;
+      const u32 flip = d[9 + 4 * i + 1] < 0 ? 0xffffffffu : 0u;      // subtract: add the complement and one
+      u32 carry = flip & 1u;
+#pragma unroll 4
+      for (int k = 0; k < L; k++) {
+        const u32 v = st.next(k) ^ flip, x = sum[k * kFinT];
+        const u32 t = x + v, u = t + carry;
+        carry = (t < x ? 1u : 0u) | (u < t ? 1u : 0u);
+        if (last) op[(i64)k * oplane] = (int32_t)u;
+        else sum[k * kFinT] = u;
       }
-      op[(i64)k * ar.plane[oid]] = (int32_t)(u32)t;
-      carry = t >> 32;
+      s0 = s1;
+      b0 = b1;
+      n0 = n1;
+    }
+    if (ns == 0) {
+      cp_async_wait<0>();
+      for (int k = 0; k < L; k++) op[(i64)k * oplane] = (int32_t)sum[k * kFinT];
     }
   }
 }
 
 // ---------------------------------------------------------------- triangular solves: fused 'col' rounding
 // desc (10 int64): CRT row0, rows (32 nrt), column c0, ncols (<= 32), eA constant, eA index (-1 none, else +
-// xe[idx]), B row tile (its column exponents), mode, base row tile 0, destination row tile 0.  One CTA per
-// group and column chunk: for each column c, mx = max over the group's rows of the CRT bit length,
-// s = mx - (32 L - 32), e_in = eA + Pe[B row tile][c], eU = e_in + s ('col' rounding, sdpvibe/batched.py:
-// 200-231); then every entry u = round(U / 2^s) goes to the destination row tiles dst0 .. dst0 + nrt - 1:
-// mode 0 stores it (exponent eU), modes 1 / 2 form the aligned difference / sum with the base row tiles
-// base0 .. (exponent eb): e2 = max(eb, eU) + 1, round(b / 2^(e2 - eb)) -/+ round(u / 2^(e2 - eU))
-// (sdpvibe/batched.py:82-92).
+// xe[idx]), B row tile (its column exponents), mode, base row tile 0, destination row tile 0.  For each column c,
+// mx = max over the group's rows of the CRT bit length, s = mx - (32 L - 32), e_in = eA + Pe[B row tile][c],
+// eU = e_in + s ('col' rounding, sdpvibe/batched.py:200-231); then every entry u = round(U / 2^s) goes to the
+// destination row tiles dst0 .. dst0 + nrt - 1: mode 0 stores it (exponent eU), modes 1 / 2 form the aligned
+// difference / sum with the base row tiles base0 .. (exponent eb): e2 = max(eb, eU) + 1, round(b / 2^(e2 - eb))
+// -/+ round(u / 2^(e2 - eU)) (sdpvibe/batched.py:82-92).
+// Columns are independent, so a group's columns are shared out over CTAs (grid y, kColSet = 8 each: one 32-byte
+// sector per row and limb), which then hold one or two entries per thread for a few row tiles; an entry's words
+// are staged in shared-memory columns.
+constexpr int kColSet = 8;
 __global__ void __launch_bounds__(256) grp_solve_round_kernel(const int32_t* __restrict__ Wd, const i64* __restrict__ bl,
                                                               int W, i64 Ntot, i64 w, int32_t* __restrict__ P,
                                                               i64 Pplane, i64* __restrict__ Pe, i64 m, int L,
                                                               const i64* __restrict__ xe,
                                                               const i64* __restrict__ desc) {
-  __shared__ i64 s_part[8][32];
-  __shared__ i64 s_su[32], s_eu[32];
+  extern __shared__ u32 cols[];
+  __shared__ i64 s_part[32][kColSet];
+  __shared__ i64 s_su[kColSet], s_eu[kColSet];
   const i64* d = desc + 10 * (i64)blockIdx.x;
-  const i64 row0 = d[0], rows = d[1], c0 = d[2], brt0 = d[8], drt0 = d[9];
-  const int ncols = (int)d[3], mode = (int)d[7];
-  const int tid = threadIdx.x, c = tid & 31, rg = tid >> 5;
+  const int cfirst = blockIdx.y * kColSet;
+  if (cfirst >= (int)d[3]) return;
+  const i64 row0 = d[0], rows = d[1], c0 = d[2] + cfirst, brt0 = d[8], drt0 = d[9];
+  const int ncols = (int)d[3] - cfirst < kColSet ? (int)d[3] - cfirst : kColSet, mode = (int)d[7];
+  const int T = blockDim.x, tid = threadIdx.x, c = tid % kColSet, rg = tid / kColSet, nrg = T / kColSet;
   i64 mx = 0;
   if (c < ncols)
-    for (i64 r = rg; r < rows; r += 8) {
+    for (i64 r = rg; r < rows; r += nrg) {
       const i64 v = bl[(row0 + r) * w + c0 + c];
       mx = v > mx ? v : mx;
     }
@@ -184,7 +226,7 @@ __global__ void __launch_bounds__(256) grp_solve_round_kernel(const int32_t* __r
   __syncthreads();
   if (tid < ncols) {
     i64 v = s_part[0][tid];
-    for (int q = 1; q < 8; q++) v = s_part[q][tid] > v ? s_part[q][tid] : v;
+    for (int q = 1; q < nrg; q++) v = s_part[q][tid] > v ? s_part[q][tid] : v;
     const i64 s = v - (32 * (i64)L - 32);
     const i64 eA = d[4] + (d[5] >= 0 ? xe[d[5]] : 0);
     s_su[tid] = s;
@@ -192,39 +234,55 @@ __global__ void __launch_bounds__(256) grp_solve_round_kernel(const int32_t* __r
   }
   __syncthreads();
   const i64 nrt = rows / 32;
-  for (i64 idx = tid; idx < rows * ncols; idx += blockDim.x) {
+  u32* cu = cols + tid;                                  // L + 3 words of U, then L of b
+  u32* cb = cu + (L + 3) * T;
+  for (i64 idx = tid; idx < rows * ncols; idx += T) {
     const int cc = (int)(idx % ncols);
     const i64 rr = idx / ncols, t = rr / 32, r = rr % 32;
     const int32_t* u = Wd + (row0 + rr) * w + c0 + cc;
-    auto uat = [&](i64 k) { return (u32)u[k * Ntot]; };
     int32_t* dst = P + (drt0 + t) * 32 * m + r * m + c0 + cc;
+    const int su = clamp_shift(s_su[cc], W, L), q = su >> 5;
+    const int b0 = q - 1 > 0 ? (q - 1 < W - 1 ? q - 1 : W - 1) : 0;
+    const int e = q + L + 1 < W ? (q + L + 1 > b0 ? q + L + 1 : b0) : W;
+    stage_col(cu, T, u + (i64)b0 * Ntot, Ntot, e - b0);
+    cp_async4(cu + (L + 2) * T, u + (i64)(W - 1) * Ntot, 4u);
+    if (mode) stage_col(cb, T, P + (brt0 + t) * 32 * m + r * m + c0 + cc, Pplane, L);
+    cp_async_commit();
+    const i64 eb = mode ? Pe[(brt0 + t) * m + c0 + cc] : 0, eu = s_eu[cc];
+    cp_async_wait<0>();
+    const u32 ext = (cu[(L + 2) * T] >> 31) ? 0xffffffffu : 0u;
+    auto st = make_shr([&](int j) { return j < 0 ? 0u : (j >= W ? ext : cu[(j - b0) * T]); }, su);
     if (mode == 0) {
-      ShiftStream st;
-      shr_begin(st, uat, W, s_su[cc]);
-      for (int k = 0; k < L; k++) dst[(i64)k * Pplane] = (int32_t)shr_next(st, uat, W, k);
+#pragma unroll 4
+      for (int k = 0; k < L; k++) dst[(i64)k * Pplane] = (int32_t)st.next(k);
       continue;
     }
-    u32 uv[kLMax];
-    shr_all(uat, W, s_su[cc], uv, L);
-    const i64 eb = Pe[(brt0 + t) * m + c0 + cc];
-    const i64 eu = s_eu[cc];
-    const i64 e2 = (eb > eu ? eb : eu) + 1;
-    const int32_t* b = P + (brt0 + t) * 32 * m + r * m + c0 + cc;
-    auto bat = [&](i64 k) { return (u32)b[k * Pplane]; };
-    auto vat = [&](i64 k) { return uv[k]; };
-    ShiftStream sb, su;
-    shr_begin(sb, bat, L, e2 - eb);
-    shr_begin(su, vat, L, e2 - eu);
-    const i64 sgn = mode == 1 ? -1 : 1;
-    i64 carry = 0;
-    u32 out[kLMax];
-    for (int k = 0; k < L; k++) {
-      const u32 x = shr_next(sb, bat, L, k), y = shr_next(su, vat, L, k);
-      const i64 tt = (i64)x + sgn * (i64)y + carry;
-      out[k] = (u32)tt;
-      carry = tt >> 32;
+    // u in place of U: for su >= 0 word k is written after index q + k + 1 - b0 > k was read (b0 is q - 1, 0 below);
+    // a left shift (nothing to round) reads at or below k, so it runs downward
+    if (su >= 0) {
+#pragma unroll 4
+      for (int k = 0; k < L; k++) {
+        const u32 v = st.next(k);
+        cu[k * T] = v;
+      }
+    } else {
+      for (int k = L - 1; k >= 0; k--) {
+        const u32 v = __funnelshift_r(st.w(q + k), st.w(q + k + 1), su & 31);
+        cu[k * T] = v;
+      }
     }
-    for (int k = 0; k < L; k++) dst[(i64)k * Pplane] = (int32_t)out[k];
+    const i64 e2 = (eb > eu ? eb : eu) + 1;
+    auto sb = make_shr(make_col(cb, T, L), clamp_shift(e2 - eb, L, L));
+    auto sv = make_shr(make_col(cu, T, L), clamp_shift(e2 - eu, L, L));
+    const u32 flip = mode == 1 ? 0xffffffffu : 0u;
+    u32 carry = flip & 1u;
+#pragma unroll 4
+    for (int k = 0; k < L; k++) {
+      const u32 x = sb.next(k), y = sv.next(k) ^ flip;
+      const u32 a = x + y, o = a + carry;
+      carry = (a < x ? 1u : 0u) | (o < a ? 1u : 0u);
+      dst[(i64)k * Pplane] = (int32_t)o;
+    }
   }
   __syncthreads();
   if (tid < ncols) {
@@ -241,111 +299,151 @@ __global__ void __launch_bounds__(256) grp_solve_round_kernel(const int32_t* __r
 
 // ---------------------------------------------------------------- triangular solves: common column exponents
 // desc (4 int64): first row tile, row tiles, column c0, ncols (<= 32).  ee[c] = max over the row tiles of
-// Pe[rt][c]; every entry is re-rounded to it (sdpvibe/batched.py:45-52) and Pe set to ee.
+// Pe[rt][c]; every entry is re-rounded to it (sdpvibe/batched.py:45-52) and Pe set to ee.  Columns shared out over
+// CTAs as in grp_solve_round.
 __global__ void __launch_bounds__(256) grp_merge_kernel(int32_t* __restrict__ P, i64 Pplane, i64* __restrict__ Pe,
                                                         i64 m, int L, const i64* __restrict__ desc) {
-  __shared__ i64 s_ee[32];
+  extern __shared__ u32 cols[];
+  __shared__ i64 s_ee[kColSet];
   const i64* d = desc + 4 * (i64)blockIdx.x;
-  const i64 rt0 = d[0], nrt = d[1], c0 = d[2];
-  const int ncols = (int)d[3];
-  if (threadIdx.x < ncols) {
-    i64 ee = Pe[rt0 * m + c0 + threadIdx.x];
+  const int cfirst = blockIdx.y * kColSet;
+  if (cfirst >= (int)d[3]) return;
+  const i64 rt0 = d[0], nrt = d[1], c0 = d[2] + cfirst;
+  const int ncols = (int)d[3] - cfirst < kColSet ? (int)d[3] - cfirst : kColSet;
+  const int T = blockDim.x, tid = threadIdx.x;
+  if (tid < ncols) {
+    i64 ee = Pe[rt0 * m + c0 + tid];
     for (i64 t = 1; t < nrt; t++) {
-      const i64 v = Pe[(rt0 + t) * m + c0 + threadIdx.x];
+      const i64 v = Pe[(rt0 + t) * m + c0 + tid];
       ee = v > ee ? v : ee;
     }
-    s_ee[threadIdx.x] = ee;
+    s_ee[tid] = ee;
   }
   __syncthreads();
+  u32* col = cols + tid;
   const i64 n = nrt * 32 * ncols;
-  for (i64 idx = threadIdx.x; idx < n; idx += blockDim.x) {
+  for (i64 idx = tid; idx < n; idx += T) {
     const int c = (int)(idx % ncols);
     const i64 rr = idx / ncols, t = rr / 32, r = rr % 32;
     const i64 s = s_ee[c] - Pe[(rt0 + t) * m + c0 + c];
     if (s == 0) continue;
     int32_t* x = P + (rt0 + t) * 32 * m + r * m + c0 + c;
-    auto at = [&](i64 k) { return (u32)x[k * Pplane]; };
-    ShiftStream st;                          // in place: word k is written after words >= k were read
-    shr_begin(st, at, L, s);
-    for (int k = 0; k < L; k++) {
-      const u32 v = shr_next(st, at, L, k);
-      x[(i64)k * Pplane] = (int32_t)v;
-    }
+    stage_col(col, T, x, Pplane, L);
+    cp_async_commit();
+    cp_async_wait<0>();
+    auto st = make_shr(make_col(col, T, L), clamp_shift(s, L, L));
+#pragma unroll 4
+    for (int k = 0; k < L; k++) x[(i64)k * Pplane] = (int32_t)st.next(k);
   }
   __syncthreads();
-  if (threadIdx.x < ncols)
-    for (i64 t = 0; t < nrt; t++) Pe[(rt0 + t) * m + c0 + threadIdx.x] = s_ee[threadIdx.x];
+  if (tid < ncols)
+    for (i64 t = 0; t < nrt; t++) Pe[(rt0 + t) * m + c0 + tid] = s_ee[tid];
 }
 
 // ---------------------------------------------------------------- base-tile conversions
+// Both work on 128 entries (4 rows) per CTA, eight CTAs per tile (grid y), with the wide, entry-major numbers passing
+// through shared memory (an odd row length WL | 1: conflict free by entry) so that global memory sees whole runs.
+constexpr int kTileT = 128;
+
 // Diagonal tile (factor arena entry base fbase[t], exponent e) -> wide fixed point (WL words, exponent -F):
 // the exact shift by e + F; entries above the diagonal are zero.  Out entry-major (tiles, 32, 32, WL).
-__global__ void __launch_bounds__(256) grp_tile_widen_kernel(const int32_t* __restrict__ Fa, i64 Fplane, int L,
-                                                             i64 e, int WL, int LF, const i64* __restrict__ fbase,
-                                                             u32* __restrict__ out) {
-  const i64 base = fbase[blockIdx.x];
+__global__ void __launch_bounds__(kTileT) grp_tile_widen_kernel(const int32_t* __restrict__ Fa, i64 Fplane, int L,
+                                                                i64 e, int WL, int LF, const i64* __restrict__ fbase,
+                                                                u32* __restrict__ out) {
+  extern __shared__ u32 cols[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, WP = WL | 1;
+  const int idx = blockIdx.y * kTileT + tid, r = idx >> 5, c = idx & 31;
+  u32* col = cols + tid;                               // L words; then the wide entries
+  u32* wide = cols + L * kTileT;
   const i64 s = -32 * (i64)LF - e;
-  for (int idx = threadIdx.x; idx < 1024; idx += blockDim.x) {
-    const int r = idx >> 5, c = idx & 31;
-    u32* o = out + ((i64)blockIdx.x * 1024 + idx) * WL;
-    if (c > r) {
-      for (int k = 0; k < WL; k++) o[k] = 0;
-      continue;
-    }
-    const int32_t* x = Fa + base + idx;
-    auto at = [&](i64 k) { return (u32)x[k * Fplane]; };
-    ShiftStream st;
-    shr_begin(st, at, L, s);
-    for (int k = 0; k < WL; k++) o[k] = shr_next(st, at, L, k);
+  u32* mine = wide + tid * WP;
+  if (c <= r) {
+    stage_col(col, kTileT, Fa + fbase[blockIdx.x] + idx, Fplane, L);
+    cp_async_commit();
+    cp_async_wait<0>();
+    auto st = make_shr(make_col(col, kTileT, L), clamp_shift(s, L, WL));
+#pragma unroll 4
+    for (int k = 0; k < WL; k++) mine[k] = st.next(k);
+  } else {
+    for (int k = 0; k < WL; k++) mine[k] = 0u;
   }
+  __syncthreads();
+  u32* o = out + ((i64)blockIdx.x * 1024 + blockIdx.y * kTileT) * WL;
+  for (int n = warp; n < kTileT; n += kTileT / 32)
+    for (int k = lane; k < WL; k += 32) o[(i64)n * WL + k] = wide[n * WP + k];
+}
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
 // Factored tile (wide, exponent -F) -> the factor arena at exponent e (L limbs, zero above the diagonal);
 // its inverse (wide) -> the inverse arena at xe = max bit length - F - (32 L - 32) over the tile (one exponent
-// per tile, sdpvibe/batched.py:243-262).
-__global__ void __launch_bounds__(256) grp_tile_narrow_kernel(const u32* __restrict__ Lw, const u32* __restrict__ Xw,
-                                                              int WL, int LF, int32_t* __restrict__ Fa, i64 Fplane,
-                                                              int L, i64 e, const i64* __restrict__ fbase,
-                                                              int32_t* __restrict__ Xa, i64 Xplane,
-                                                              const i64* __restrict__ xidx, i64* __restrict__ xe) {
-  __shared__ int s_max[8];
-  const i64 F = 32 * (i64)LF;
+// per tile, sdpvibe/batched.py:243-262): the eight CTAs of a tile form a cluster and exchange their maxima.
+__global__ void __cluster_dims__(1, 8, 1) __launch_bounds__(kTileT)
+    grp_tile_narrow_kernel(const u32* __restrict__ Lw, const u32* __restrict__ Xw, int WL, int LF,
+                           int32_t* __restrict__ Fa, i64 Fplane, int L, i64 e, const i64* __restrict__ fbase,
+                           int32_t* __restrict__ Xa, i64 Xplane, const i64* __restrict__ xidx, i64* __restrict__ xe) {
+  extern __shared__ u32 cols[];
+  __shared__ int s_max[kTileT / 32], s_all;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, WP = WL | 1;
+  const int idx = blockIdx.y * kTileT + tid, r = idx >> 5, c = idx & 31;
+  const i64 F = 32 * (i64)LF, first = ((i64)blockIdx.x * 1024 + blockIdx.y * kTileT) * WL;
   const i64 base = fbase[blockIdx.x], xi = xidx[blockIdx.x];
-  int mx = 0;
-  for (int idx = threadIdx.x; idx < 1024; idx += blockDim.x) {
-    const int r = idx >> 5, c = idx & 31;
-    const u32* lw = Lw + ((i64)blockIdx.x * 1024 + idx) * WL;
-    int32_t* fo = Fa + base + idx;
-    if (c > r) {
-      for (int k = 0; k < L; k++) fo[(i64)k * Fplane] = 0;
-    } else {
-      auto at = [&](i64 k) { return lw[k]; };
-      ShiftStream st;
-      shr_begin(st, at, WL, e + F);
-      for (int k = 0; k < L; k++) fo[(i64)k * Fplane] = (int32_t)shr_next(st, at, WL, k);
+  u32 *wl = cols, *wx = cols + kTileT * WP;
+  for (int n = warp; n < kTileT; n += kTileT / 32)
+    for (int k = lane; k < WL; k += 32) {
+      cp_async4(wx + n * WP + k, Xw + first + (i64)n * WL + k, 4u);
+      cp_async4(wl + n * WP + k, Lw + first + (i64)n * WL + k, 4u);
     }
-    const int b = bitlen_words(Xw + ((i64)blockIdx.x * 1024 + idx) * WL, WL);
-    mx = b > mx ? b : mx;
-  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  const u32 *myl = wl + tid * WP, *myx = wx + tid * WP;
+  int mx = col_bits(myx, 1, WL);
   for (int o = 16; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
+  if (lane == 0) s_max[warp] = mx;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    int v = threadIdx.x < (blockDim.x >> 5) ? s_max[threadIdx.x] : 0;
-    for (int o = 16; o; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (threadIdx.x == 0) s_max[0] = v;
+  if (tid == 0) s_all = max(max(s_max[0], s_max[1]), max(s_max[2], s_max[3]));
+  cluster_sync();
+  int tile_max = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    u32 addr;
+    int v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(&s_all)), "r"(k));
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr));
+    tile_max = max(tile_max, v);
   }
-  __syncthreads();
-  const i64 ex = (i64)s_max[0] - F - (32 * (i64)L - 32);
-  for (int idx = threadIdx.x; idx < 1024; idx += blockDim.x) {
-    const u32* xw = Xw + ((i64)blockIdx.x * 1024 + idx) * WL;
-    auto at = [&](i64 k) { return xw[k]; };
-    ShiftStream st;
-    shr_begin(st, at, WL, ex + F);
-    int32_t* xo = Xa + xi * 1024 + idx;
-    for (int k = 0; k < L; k++) xo[(i64)k * Xplane] = (int32_t)shr_next(st, at, WL, k);
+  cluster_sync();
+  int32_t* fo = Fa + base + idx;
+  if (c > r) {
+    for (int k = 0; k < L; k++) fo[(i64)k * Fplane] = 0;
+  } else {
+    auto st = make_shr(make_col(myl, 1, WL), clamp_shift(e + F, WL, L));
+#pragma unroll 4
+    for (int k = 0; k < L; k++) fo[(i64)k * Fplane] = (int32_t)st.next(k);
   }
-  if (threadIdx.x == 0) xe[xi] = ex;
+  const i64 ex = (i64)tile_max - F - (32 * (i64)L - 32);
+  auto sx = make_shr(make_col(myx, 1, WL), clamp_shift(ex + F, WL, L));
+  int32_t* xo = Xa + xi * 1024 + idx;
+#pragma unroll 4
+  for (int k = 0; k < L; k++) xo[(i64)k * Xplane] = (int32_t)sx.next(k);
+  if (tid == 0 && blockIdx.y == 0) xe[xi] = ex;
+}
+
+// Dynamic shared memory of `bytes`, the kernel's limit raised to the most a CTA can have, once per device.
+template <class Kernel>
+int grp_smem(Kernel kernel, size_t bytes, bool (&set)[64]) {
+  if (bytes > 220 * 1024) return SDPV_EINVAL;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!set[dev & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    if (e != cudaSuccess) return sdpv::set_cuda_error(e);
+    set[dev & 63] = true;
+  }
+  return SDPV_OK;
 }
 
 Arenas make_arenas(int32_t* const* ptrs, const int64_t* planes, int n) {
@@ -378,7 +476,11 @@ extern "C" int sdpv_grp_finish_fixed(const int32_t* Wd, int W, int64_t Ntot, int
       ndesc > 0x7fffffff || (ndesc && !desc))
     return SDPV_EINVAL;
   if (ndesc == 0) return SDPV_OK;
-  grp_finish_fixed_kernel<<<dim3((unsigned)ndesc, 4), 256, 0, sdpv::as_stream(stream)>>>(
+  static bool set[64] = {};
+  const size_t smem = (size_t)(L + 2 * (L + 3)) * kFinT * 4;
+  const int rc = grp_smem(grp_finish_fixed_kernel, smem, set);
+  if (rc != SDPV_OK) return rc;
+  grp_finish_fixed_kernel<<<dim3((unsigned)ndesc, 8), kFinT, smem, sdpv::as_stream(stream)>>>(
       Wd, W, Ntot, w, make_arenas(ar_host, planes_host, nar), L, xe, desc);
   return sdpv::launch_status();
 }
@@ -390,8 +492,14 @@ extern "C" int sdpv_grp_solve_round(const int32_t* Wd, const int64_t* bl, int W,
       (ndesc && !desc))
     return SDPV_EINVAL;
   if (ndesc == 0) return SDPV_OK;
-  grp_solve_round_kernel<<<(unsigned)ndesc, 256, 0, sdpv::as_stream(stream)>>>(Wd, bl, W, Ntot, w, P, Pplane, Pe, m, L,
-                                                                                xe, desc);
+  static bool set[64] = {};
+  const int T = L <= 64 ? 256 : 128;
+  const size_t smem = (size_t)(2 * L + 3) * T * 4;
+  const int rc = grp_smem(grp_solve_round_kernel, smem, set);
+  if (rc != SDPV_OK) return rc;
+  const unsigned sets = (unsigned)(((m < 32 ? m : 32) + kColSet - 1) / kColSet);
+  grp_solve_round_kernel<<<dim3((unsigned)ndesc, sets), T, smem, sdpv::as_stream(stream)>>>(Wd, bl, W, Ntot, w, P, Pplane,
+                                                                                          Pe, m, L, xe, desc);
   return sdpv::launch_status();
 }
 
@@ -399,7 +507,13 @@ extern "C" int sdpv_grp_merge(int32_t* P, int64_t Pplane, int64_t* Pe, int64_t m
                               int64_t ndesc, void* stream) {
   if (!P || !Pe || m < 1 || L < 1 || ndesc < 0 || ndesc > 0x7fffffff || (ndesc && !desc)) return SDPV_EINVAL;
   if (ndesc == 0) return SDPV_OK;
-  grp_merge_kernel<<<(unsigned)ndesc, 256, 0, sdpv::as_stream(stream)>>>(P, Pplane, Pe, m, L, desc);
+  static bool set[64] = {};
+  const int T = L <= 128 ? 256 : 128;
+  const size_t smem = (size_t)L * T * 4;
+  const int rc = grp_smem(grp_merge_kernel, smem, set);
+  if (rc != SDPV_OK) return rc;
+  const unsigned sets = (unsigned)(((m < 32 ? m : 32) + kColSet - 1) / kColSet);
+  grp_merge_kernel<<<dim3((unsigned)ndesc, sets), T, smem, sdpv::as_stream(stream)>>>(P, Pplane, Pe, m, L, desc);
   return sdpv::launch_status();
 }
 
@@ -407,7 +521,12 @@ extern "C" int sdpv_grp_tile_widen(const int32_t* Fa, int64_t Fplane, int L, int
                                    const int64_t* fbase, int64_t ntiles, uint32_t* out, void* stream) {
   if (!Fa || !fbase || !out || L < 1 || WL <= L || LF < 2 || ntiles < 0 || ntiles > 0x7fffffff) return SDPV_EINVAL;
   if (ntiles == 0) return SDPV_OK;
-  grp_tile_widen_kernel<<<(unsigned)ntiles, 256, 0, sdpv::as_stream(stream)>>>(Fa, Fplane, L, e, WL, LF, fbase, out);
+  static bool set[64] = {};
+  const size_t smem = (size_t)(L + (WL | 1)) * kTileT * 4;
+  const int rc = grp_smem(grp_tile_widen_kernel, smem, set);
+  if (rc != SDPV_OK) return rc;
+  grp_tile_widen_kernel<<<dim3((unsigned)ntiles, 8), kTileT, smem, sdpv::as_stream(stream)>>>(Fa, Fplane, L, e, WL, LF,
+                                                                                             fbase, out);
   return sdpv::launch_status();
 }
 
@@ -418,7 +537,11 @@ extern "C" int sdpv_grp_tile_narrow(const uint32_t* Lw, const uint32_t* Xw, int 
       ntiles > 0x7fffffff)
     return SDPV_EINVAL;
   if (ntiles == 0) return SDPV_OK;
-  grp_tile_narrow_kernel<<<(unsigned)ntiles, 256, 0, sdpv::as_stream(stream)>>>(Lw, Xw, WL, LF, Fa, Fplane, L, e, fbase,
-                                                                                  Xa, Xplane, xidx, xe);
+  static bool set[64] = {};
+  const size_t smem = (size_t)2 * (WL | 1) * kTileT * 4;
+  const int rc = grp_smem(grp_tile_narrow_kernel, smem, set);
+  if (rc != SDPV_OK) return rc;
+  grp_tile_narrow_kernel<<<dim3((unsigned)ntiles, 8), kTileT, smem, sdpv::as_stream(stream)>>>(
+      Lw, Xw, WL, LF, Fa, Fplane, L, e, fbase, Xa, Xplane, xidx, xe);
   return sdpv::launch_status();
 }
