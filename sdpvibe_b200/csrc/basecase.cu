@@ -171,14 +171,14 @@ __device__ __forceinline__ void warp_negate(u32 (&v)[NPL], int WL) {
 
 template <int NPL>
 __device__ __forceinline__ int warp_top(const u32 (&v)[NPL], int WL) {
+  // one warp reduction, whose result the compiler knows to be the same in every lane: the loops bounded by it need
+  // no reconvergence
   const int lane = threadIdx.x & 31;
-  int top = 0;
+  unsigned top = 0;
 #pragma unroll
-  for (int c = 0; c < NPL; c++) {
-    const unsigned b = __ballot_sync(kFull, lane + 32 * c < WL && v[c] != 0);
-    if (b) top = 32 * c + 31 - __clz(b);
-  }
-  return top;
+  for (int c = 0; c < NPL; c++)
+    if (lane + 32 * c < WL && v[c] != 0) top = lane + 32 * c;
+  return (int)__reduce_max_sync(kFull, top);
 }
 
 // Magnitude of a two's-complement WL-word operand (shared or global memory) into m[0..WL); returns its sign,
@@ -186,7 +186,7 @@ __device__ __forceinline__ int warp_top(const u32 (&v)[NPL], int WL) {
 template <int NPL>
 __device__ __forceinline__ int load_mag(const u32* src, u32* m, int WL, int& top) {
   const int lane = threadIdx.x & 31;
-  const int sign = (int)(src[WL - 1] >> 31);
+  const int sign = __any_sync(kFull, src[WL - 1] >> 31) ? 1 : 0;
   u32 v[NPL];
 #pragma unroll
   for (int c = 0; c < NPL; c++) v[c] = lane + 32 * c < WL ? src[lane + 32 * c] : 0u;
@@ -202,9 +202,7 @@ __device__ __forceinline__ int load_mag(const u32* src, u32* m, int WL, int& top
 // tops tx, ty): one product column per lane, columns kmin .. min(kmax + 2, LF + WL - 1), each a 96-bit exact
 // sum; the column sums are added with their 32- and 64-bit shifts and the carries resolved by chain_carry.
 // x, y: shared memory (read at words <= their tops); out: 32 NPL words of shared memory, overwritten.
-// SQ: a square (y = x, ty = tx): each column sums the products x_i x_(k-i), i < k - i, doubles the sum and
-// adds the middle term x_(k/2)^2 (half the multiply-adds, the same exact column sums).
-template <int NPL, bool SQ = false>
+template <int NPL>
 __device__ void wmul_core(const u32* x, int tx, const u32* y, int ty, int t, int WL, int LF, u32* out) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -221,8 +219,7 @@ __device__ void wmul_core(const u32* x, int tx, const u32* y, int ty, int t, int
     u32 c0 = 0, c1 = 0, c2 = 0;
     {
       const bool act = q < ncol && k <= kmax;
-      const int i0 = max(la, k - ty), i1f = act ? min(tx, k - lb) : i0 - 1;
-      const int i1 = SQ ? min(i1f, (k - 1) >> 1) : i1f;          // SQ: the pairs i < k - i
+      const int i0 = max(la, k - ty), i1 = act ? min(tx, k - lb) : i0 - 1;
       const int nt = (int)__reduce_max_sync(kFull, (unsigned)max(i1 - i0 + 1, 0));
       u32 d0 = 0, d1 = 0, d2 = 0, e0 = 0, e1 = 0, e2 = 0, f0 = 0, f1 = 0, f2 = 0;
       // the next four terms' loads are issued before this four's multiply-adds (software pipelined)
@@ -254,13 +251,6 @@ __device__ void wmul_core(const u32* x, int tx, const u32* y, int ty, int t, int
       add96(d0, d1, d2, f0, f1, f2);
       add96(c0, c1, c2, e0, e1, e2);
       add96(c0, c1, c2, d0, d1, d2);
-      if (SQ) {
-        c2 = (c2 << 1) | (c1 >> 31);
-        c1 = (c1 << 1) | (c0 >> 31);
-        c0 <<= 1;
-        const int mid = k >> 1;
-        if (!(k & 1) && i0 <= mid && mid <= i1f) mac96(c0, c1, c2, x[mid], x[mid]);
-      }
     }
     u32 c1u = __shfl_up_sync(kFull, c1, 1), c2u = __shfl_up_sync(kFull, c2, 2);
     if (lane == 0) c1u = p_c1;
@@ -285,6 +275,95 @@ __device__ void wmul_core(const u32* x, int tx, const u32* y, int ty, int t, int
   }
   __syncwarp();
 }
+
+// ---- the latency-critical product: the same truncated product as wmul_core with the result left in registers
+// (word lane + 32 c in m[c]) and no bounds in its inner loop.  Every lane runs the same x words la .. tx (uniform
+// 16-byte loads) against y[k - i] of its own column k, read from a padded buffer whose words outside y's kept
+// range are zero; a run of lanes reads consecutive words.  Against wmul_core (per-lane term ranges, predicated
+// loads, the result through shared memory): 32 x 32 tile factor at L = 26 383 -> 342 us (17
+// products per pivot on its critical path), inverse 244 -> 231 us; of that 15 us from tops and signs taken by
+// reductions and votes, whose uniform results keep reconvergence out of the loops and branches they bound.
+// Words go in groups of four, the next group's loads issued ahead of this group's multiply-adds.  Groups of
+// eight (398 us) and one call site for the Newton chain's three products (410-456 us) were slower.
+//   x: 16-byte aligned, zero from tx + 1 to the end of tx's group of four and below la within la's group
+//   y: word 0 of a padded buffer (kPadLo / kPadHi), zero below lb and above ty
+template <int NPL>
+constexpr int kPadLo = 32 * NPL + 8;             // lowest index read: -(32 NPL + 6)
+template <int NPL>
+constexpr int kPadHi = 64 * NPL;                 // highest: kmax = tx + ty
+template <int NPL>
+constexpr int kPadWords = kPadLo<NPL> + kPadHi<NPL>;
+
+template <int NPL>
+__device__ __forceinline__ void wmul_pad(const u32* x, int tx, int la, const u32* y, int ty, int lb, int LF,
+                                         u32 (&m)[NPL]) {
+  const int lane = threadIdx.x & 31;
+  const int kmin = max(LF - 2, la + lb), kmax = tx + ty;
+  const int ncol = kmax + 2 - kmin + 1, ibase = la & ~3, ng = (tx >> 2) - (la >> 2) + 1;
+#pragma unroll
+  for (int c = 0; c < NPL; c++) m[c] = 0u;
+  u32 p_c1 = 0, p_c2a = 0, p_c2b = 0, p_h = 0, cin = 0;          // carried over from the previous 32 columns
+  for (int q0 = 0; q0 < ncol; q0 += 32) {
+    const int k = kmin + q0 + lane, kc = min(k, kmax);
+    const u32* p = y + (kc - ibase);
+    const uint4* xp = reinterpret_cast<const uint4*>(x + ibase);
+    u32 c0 = 0, c1 = 0, c2 = 0, d0 = 0, d1 = 0, d2 = 0;
+    uint4 xv = *xp;
+    u32 y0 = p[0], y1 = p[-1], y2 = p[-2], y3 = p[-3];
+#pragma unroll 2
+    for (int g = 0; g < ng; g++) {
+      const uint4 xn = xp[g + 1];                                // (one group past the end is read, unused)
+      p -= 4;
+      const u32 n0 = p[0], n1 = p[-1], n2 = p[-2], n3 = p[-3];
+      mac96(c0, c1, c2, xv.x, y0);
+      mac96(d0, d1, d2, xv.y, y1);
+      mac96(c0, c1, c2, xv.z, y2);
+      mac96(d0, d1, d2, xv.w, y3);
+      xv = xn;
+      y0 = n0;
+      y1 = n1;
+      y2 = n2;
+      y3 = n3;
+    }
+    add96(c0, c1, c2, d0, d1, d2);
+    if (k > kmax) c0 = c1 = c2 = 0;
+    u32 c1u = __shfl_up_sync(kFull, c1, 1), c2u = __shfl_up_sync(kFull, c2, 2);
+    if (lane == 0) c1u = p_c1;
+    if (lane == 0) c2u = p_c2a;
+    if (lane == 1) c2u = p_c2b;
+    const u64 v = (u64)c0 + c1u + c2u;                                 // < 3 * 2^32
+    const u32 lo = (u32)v, h = (u32)(v >> 32);
+    u32 hu = __shfl_up_sync(kFull, h, 1);
+    if (lane == 0) hu = p_h;
+    const u32 e = lo + hu;
+    u32 cout;
+    const u32 w = e + chain_carry(e < lo, e == kFull, cin, cout);      // column k's word
+#pragma unroll
+    for (int c = 0; c < NPL; c++) {
+      const int q = lane + 32 * c + LF - kmin - q0;                    // the lane that holds result word lane + 32 c
+      const u32 r = __shfl_sync(kFull, w, q & 31);
+      if ((unsigned)q < 32u) m[c] = r;                                 // (columns past kmax + 2 are zero)
+    }
+    if (q0 + 32 < ncol) {
+      p_c1 = __shfl_sync(kFull, c1, 31);
+      p_c2a = __shfl_sync(kFull, c2, 30);
+      p_c2b = __shfl_sync(kFull, c2, 31);
+      p_h = __shfl_sync(kFull, h, 31);
+      cin = cout;
+    }
+  }
+}
+template <int NPL>
+__device__ __forceinline__ void clip_words(u32 (&v)[NPL], int WL) {    // zero at and above WL
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int c = 0; c < NPL; c++)
+    if (lane + 32 * c >= WL) v[c] = 0u;
+}
+// a value that every lane read alike (shared memory), made one the compiler knows to be uniform
+__device__ __forceinline__ int uniform_top(int top) { return (int)__reduce_max_sync(kFull, (unsigned)top); }
+// first word of an operand of top `top` kept by a product that takes the top t words (t = 0: all)
+__device__ __forceinline__ int first_kept(int top, int t) { return t ? max(0, top - t + 1) : 0; }
 
 // The truncated product a * b >> F of two's-complement operands (magnitudes multiplied by wmul_core, sign
 // applied last).  Outputs (any may be null): out = signed result (may alias a or b), omag = magnitude,
@@ -335,6 +414,13 @@ __device__ __forceinline__ void reg_store(u32* dst, const u32 (&v)[NPL], int WL)
   for (int c = 0; c < NPL; c++)
     if (lane + 32 * c < WL) dst[lane + 32 * c] = v[c];
 }
+// all 32 NPL words (zero at and above WL), those below lo as zero
+template <int NPL>
+__device__ __forceinline__ void reg_store_from(u32* dst, const u32 (&v)[NPL], int lo) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int c = 0; c < NPL; c++) dst[lane + 32 * c] = lane + 32 * c >= lo ? v[c] : 0u;
+}
 // word w of v, in every lane
 template <int NPL>
 __device__ __forceinline__ u32 reg_word(const u32 (&v)[NPL], int w) {
@@ -345,6 +431,15 @@ __device__ __forceinline__ u32 reg_word(const u32 (&v)[NPL], int w) {
     if (c == (w >> 5)) r = x;
   }
   return r;
+}
+// sign of v, the same in every lane and known to be (a vote): branches on it need no reconvergence
+template <int NPL>
+__device__ __forceinline__ bool reg_sign(const u32 (&v)[NPL], int WL) {
+  const int lane = threadIdx.x & 31;
+  bool s = false;
+#pragma unroll
+  for (int c = 0; c < NPL; c++) s = s || (lane + 32 * c == WL - 1 && (v[c] >> 31));
+  return __any_sync(kFull, s);
 }
 // r = a + b or a - b (mod 2^(32 WL)); r may alias a or b
 template <int NPL>
@@ -662,14 +757,47 @@ __device__ __forceinline__ void warp_shr1(u32* x, int WL) {              // arit
 __host__ __device__ constexpr int pitch(int WL) { return WL | 1; }
 template <int NPL, bool GLOBAL>
 __host__ __device__ constexpr size_t chol_smem_bytes(int WL) {
-  return (size_t)((GLOBAL ? 0 : 528) + 32) * pitch(WL) * 4 + kWarpsS * sizeof(WarpScratchT<NPL>) + 6 * 32 * NPL * 4 + 80;
+  return (size_t)((GLOBAL ? 0 : 528) + 32) * pitch(WL) * 4 + 16 + kWarpsS * sizeof(WarpScratchT<NPL>) +
+         (4 * 32 * NPL + 4 + 4 * kPadWords<NPL>) * 4 + 80;
 }
 template <int NPL, bool GLOBAL>
 __host__ __device__ constexpr size_t trinv_smem_bytes(int WL) {
-  return (size_t)((GLOBAL ? 0 : 528) + 96) * pitch(WL) * 4 + kWarpsS * sizeof(WarpScratchT<NPL>) + 2 * 528 + 128 + 64;
+  return (size_t)((GLOBAL ? 0 : 528) + 64) * pitch(WL) * 4 + 16 + kWarpsS * sizeof(WarpScratchT<NPL>) +
+         2 * kPadWords<NPL> * 4 + 2 * 528 + 128 + 64;
 }
 
 __device__ __forceinline__ int tri(int i, int j) { return i * (i + 1) / 2 + j; }
+
+// The Newton schedule on whatever d holds (zero, negative: the error word is set, the words still follow the
+// reference); out of line, so that it does not lie between the chain's instructions.  One warp; |r| left in sr.
+template <int NPL>
+__device__ __noinline__ void newton_any(const u32* sd, u32* sr, u32* st1, u32* st2, const u32* sone, u32* rout, int* info,
+                                        int WL, int LF, WarpScratchT<NPL>& ws) {
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) fx_from_double(sr, 1.0 / sqrt(fx_to_double(sd, WL, LF)), WL, LF);
+  __syncwarp();
+  for (int bits = 100;; bits *= 2) {                             // r <- r + r (1 - d r^2) / 2
+    int t = bits / 32 + 2;
+    if (t >= WL) t = 0;
+    wmul<NPL>(sr, sr, t, WL, LF, ws, st1, nullptr, nullptr, nullptr);
+    wmul<NPL>(st1, sd, t, WL, LF, ws, st2, nullptr, nullptr, nullptr);
+    warp_addsub<NPL>(st1, sone, st2, true, WL);
+    wmul<NPL>(sr, st1, t, WL, LF, ws, st2, nullptr, nullptr, nullptr);
+    warp_shr1<NPL>(st2, WL);
+    warp_addsub<NPL>(sr, sr, st2, false, WL);
+    if (t == 0) break;
+  }
+  for (int w = lane; w < WL; w += 32) rout[w] = sr[w];
+  int tr;
+  const int sg = load_mag<NPL>(sr, st2, WL, tr);                // |r|, then back into sr
+  __syncwarp();
+  for (int w = lane; w < WL; w += 32) sr[w] = st2[w];
+  if (lane == 0) {
+    info[0] = tr;
+    info[2] = sg;
+  }
+  __syncwarp();
+}
 
 // NPL words per lane (WL <= 32 NPL); GLOBAL: the working triangle is the tile itself in global memory (entry
 // (i, j) at (32 i + j) WL), else a copy in shared memory (entry (i, j) at tri(i, j), odd pitch WP).
@@ -684,12 +812,17 @@ __global__ void __launch_bounds__(kThreadsS) chol_tiles_k(u32* __restrict__ A, u
     return GLOBAL ? G + ((size_t)i * BT + j) * WL : T + tri(i, j) * WP;
   };
   u32* colmag = GLOBAL ? sm : sm + 528 * WP;                     // |l_ik| of the current column
-  WarpScratchT<NPL>* ws = reinterpret_cast<WarpScratchT<NPL>*>(colmag + 32 * WP);
+  WarpScratchT<NPL>* ws = reinterpret_cast<WarpScratchT<NPL>*>(((uintptr_t)(colmag + 32 * WP) + 15) & ~(uintptr_t)15);
   u32* nw = reinterpret_cast<u32*>(ws + kWarpsS);
-  // |r| of pivots of alternate parity in rbuf[k & 1]: warp 0 runs pivot k + 1 while the other warps still scale
-  // column k by r_k
-  u32 *sd = nw, *st1 = nw + NWD, *st2 = nw + 2 * NWD, *sone = nw + 3 * NWD, *rbuf = nw + 4 * NWD;
-  uint8_t* colsign = reinterpret_cast<uint8_t*>(nw + 6 * NWD);
+  // warp 0's scratch: words of the general path (sd, st1, st2, sone); xs: the unpadded operand of its products;
+  // padded operands: rm (r, or the row whose square is taken), dm (d), and |r| of pivots of alternate parity in
+  // rpad(k & 1): warp 0 runs pivot k + 1 while the other warps still scale column k by r_k
+  u32 *sd = nw, *st1 = nw + NWD, *st2 = nw + 2 * NWD, *sone = nw + 3 * NWD, *pads = nw + 4 * NWD + 4;
+  u32* xs = st1;
+  auto pad = [&](int q) { return pads + q * kPadWords<NPL> + kPadLo<NPL>; };
+  u32 *rm = pad(0), *dm = pad(1);
+  auto rpad = [&](int k) { return pad(2 + (k & 1)); };
+  uint8_t* colsign = reinterpret_cast<uint8_t*>(pads + 4 * kPadWords<NPL>);
   uint8_t* coltop = colsign + 32;
   int* rinfo = reinterpret_cast<int*>(coltop + 32);               // top and sign of |r| per parity
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -720,22 +853,19 @@ __global__ void __launch_bounds__(kThreadsS) chol_tiles_k(u32* __restrict__ A, u
         }
     }
   };
-  // Pivot k (warp 0): r = d^-1/2 by the Newton schedule; |r| in rbuf[k & 1] (top, sign in rinfo), r in RINV.
+  // Pivot k (warp 0): r = d^-1/2 by the Newton schedule; |r| in rpad(k) (top, sign in rinfo), r in RINV.
   // l_kk = d r is formed later by another warp (kkprod), off the chain of pivots.
-  auto pivot = [&](int k, const u32* akk) {                      // akk: where d = a_kk is read
-    u32* sr = rbuf + (k & 1) * NWD;
-    u32 D[NPL];
-    reg_load<NPL>(akk, D, WL);
-    reg_store<NPL>(sd, D, WL);
-    const bool dneg = reg_word<NPL>(D, WL - 1) >> 31;
+  auto pivot = [&](int k, const u32 (&D)[NPL]) {                 // D: d = a_kk
+    u32* sr = rpad(k);
+    const bool dneg = reg_sign<NPL>(D, WL);
     bool dnz = false;
 #pragma unroll
     for (int c = 0; c < NPL; c++) dnz = dnz || __any_sync(kFull, D[c] != 0u);
     if (lane == 0 && (dneg || !dnz)) atomicOr(err, SDPV_ERRBIT_NOTSPD);
     if (!dneg && dnz) {
-      // d > 0: the same truncated products as below, with the operands kept as magnitudes in shared memory
-      // (|r| in sr, d in sd, |1 - d r^2| in ws[0].xa) and the additions, sign changes and halvings done in
-      // registers; r stays positive in practice, its sign is carried all the same.  The first r is
+      // d > 0: the same truncated products as newton_any's (wmul_pad), r, 1 - d r^2 and their sums, sign changes
+      // and halvings in registers; an operand is stored once per product it enters, its words below the kept ones
+      // as zeros.  r stays positive in practice, its sign is carried all the same.  The first r is
       // fx_from_double(1 / sqrt(fx_to_double(d))), evaluated by every lane on d's top three words.
       const int td = warp_top<NPL>(D, WL);
       const u32 x0 = reg_word<NPL>(D, td), x1 = reg_word<NPL>(D, max(td - 1, 0)), x2 = reg_word<NPL>(D, max(td - 2, 0));
@@ -767,39 +897,46 @@ __global__ void __launch_bounds__(kThreadsS) chol_tiles_k(u32* __restrict__ A, u
         O[c] = (lane + 32 * c == LF) ? 1u : 0u;                   // fixed-point 1
         R[c] = Rt[c];
       }
-      u32 sR = reg_word<NPL>(Rt, WL - 1) >> 31;
+      bool sR = reg_sign<NPL>(Rt, WL);
       if (sR) warp_negate<NPL>(R, WL);
-      reg_store<NPL>(sr, R, WL);
-      __syncwarp();
       int tr = warp_top<NPL>(R, WL);
       for (int bits = 100;; bits *= 2) {                           // r <- r + r (1 - d r^2) / 2
         int t = bits / 32 + 2;
         if (t >= WL) t = 0;
-        wmul_core<NPL, true>(sr, tr, sr, tr, t, WL, LF, st1);     // r^2
-        reg_load<NPL>(st1, P, WL);
-        const int tp = warp_top<NPL>(P, WL);
-        wmul_core<NPL>(st1, tp, sd, td, t, WL, LF, st2);          // d r^2
-        reg_load<NPL>(st2, P, WL);
-        reg_addsub<NPL>(S, O, P, true, WL);                        // 1 - d r^2
-        const u32 sS = reg_word<NPL>(S, WL - 1) >> 31;
-        if (sS) warp_negate<NPL>(S, WL);
-        const int ts = warp_top<NPL>(S, WL);
-        reg_store<NPL>(ws[0].xa, S, WL);
+        const int lr = first_kept(tr, t), ld = first_kept(td, t);
+        reg_store_from<NPL>(rm, R, lr);
+        reg_store_from<NPL>(dm, D, ld);
         __syncwarp();
-        wmul_core<NPL>(sr, tr, ws[0].xa, ts, t, WL, LF, st2);     // |r (1 - d r^2)|
-        reg_load<NPL>(st2, P, WL);
-        if (sR ^ sS) warp_negate<NPL>(P, WL);
+        wmul_pad<NPL>(rm, tr, lr, rm, tr, lr, LF, P);              // r^2
+        clip_words<NPL>(P, WL);
+        const int tp = warp_top<NPL>(P, WL), lp = first_kept(tp, t);
+        reg_store_from<NPL>(xs, P, lp);
+        __syncwarp();
+        wmul_pad<NPL>(xs, tp, lp, dm, td, ld, LF, P);              // d r^2
+        clip_words<NPL>(P, WL);
+        reg_addsub<NPL>(S, O, P, true, WL);                        // 1 - d r^2
+        const bool sS = reg_sign<NPL>(S, WL);
+        if (sS) warp_negate<NPL>(S, WL);
+        clip_words<NPL>(S, WL);
+        const int ts = warp_top<NPL>(S, WL), ls = first_kept(ts, t);
+        __syncwarp();
+        reg_store_from<NPL>(xs, S, ls);
+        __syncwarp();
+        wmul_pad<NPL>(xs, ts, ls, rm, tr, lr, LF, P);              // |r (1 - d r^2)|
+        clip_words<NPL>(P, WL);
+        if (sR != sS) warp_negate<NPL>(P, WL);
         reg_shr1<NPL>(P, WL);                                      // floor of half
         reg_addsub<NPL>(Rt, Rt, P, false, WL);
-        sR = reg_word<NPL>(Rt, WL - 1) >> 31;
+        sR = reg_sign<NPL>(Rt, WL);
 #pragma unroll
         for (int c = 0; c < NPL; c++) R[c] = Rt[c];
         if (sR) warp_negate<NPL>(R, WL);
+        clip_words<NPL>(R, WL);
         tr = warp_top<NPL>(R, WL);
-        reg_store<NPL>(sr, R, WL);
-        __syncwarp();
         if (t == 0) break;
+        __syncwarp();
       }
+      reg_store_from<NPL>(sr, R, 0);
       reg_store<NPL>(RI + (size_t)k * WL, Rt, WL);
       if (lane == 0) {
         rinfo[k & 1] = tr;
@@ -807,65 +944,49 @@ __global__ void __launch_bounds__(kThreadsS) chol_tiles_k(u32* __restrict__ A, u
       }
       __syncwarp();
     } else {
+      reg_store<NPL>(sd, D, WL);
       for (int w = lane; w < WL; w += 32) sone[w] = (w == LF) ? 1u : 0u;
       __syncwarp();
-      if (lane == 0) fx_from_double(sr, 1.0 / sqrt(fx_to_double(sd, WL, LF)), WL, LF);
-      __syncwarp();
-      for (int bits = 100;; bits *= 2) {                           // r <- r + r (1 - d r^2) / 2
-        int t = bits / 32 + 2;
-        if (t >= WL) t = 0;
-        wmul<NPL>(sr, sr, t, WL, LF, ws[0], st1, nullptr, nullptr, nullptr);
-        wmul<NPL>(st1, sd, t, WL, LF, ws[0], st2, nullptr, nullptr, nullptr);
-        warp_addsub<NPL>(st1, sone, st2, true, WL);
-        wmul<NPL>(sr, st1, t, WL, LF, ws[0], st2, nullptr, nullptr, nullptr);
-        warp_shr1<NPL>(st2, WL);
-        warp_addsub<NPL>(sr, sr, st2, false, WL);
-        if (t == 0) break;
-      }
-      for (int w = lane; w < WL; w += 32) RI[(size_t)k * WL + w] = sr[w];
-      int tr;
-      const int sg = load_mag<NPL>(sr, st2, WL, tr);              // |r|, then back into sr
-      __syncwarp();
-      for (int w = lane; w < WL; w += 32) sr[w] = st2[w];
-      if (lane == 0) {
-        rinfo[k & 1] = tr;
-        rinfo[2 + (k & 1)] = sg;
-      }
-      __syncwarp();
+      newton_any<NPL>(sd, sr, st1, st2, sone, RI + (size_t)k * WL, rinfo + (k & 1), WL, LF, ws[0]);
     }
   };
-  // a (shared or global memory, may alias out) times r_k given as |r_k| in rbuf with its top and sign: the
-  // truncated product of wmul with the second operand's magnitude already formed
-  auto mul_r = [&](u32* a, int k, u32* out, u32* omag, uint8_t* osign, uint8_t* otop) {
+  // a (shared or global memory, may alias out) times r_k given as |r_k| in rpad(k) with its top and sign; the
+  // magnitude stays in m
+  auto mul_r = [&](u32* a, int k, u32* out, u32* omag, uint8_t* osign, uint8_t* otop, u32 (&m)[NPL]) {
     WarpScratchT<NPL>& s = ws[warp];
     int ta;
     const int sa = load_mag<NPL>(a, s.xa, WL, ta);
     __syncwarp();
-    wmul_core<NPL>(s.xa, ta, rbuf + (k & 1) * NWD, rinfo[k & 1], 0, WL, LF, s.acc);
-    u32 m[NPL];
-#pragma unroll
-    for (int c = 0; c < NPL; c++) m[c] = lane + 32 * c < WL ? s.acc[lane + 32 * c] : 0u;
-    const int sg = sa ^ rinfo[2 + (k & 1)];
+    wmul_pad<NPL>(s.xa, ta, 0, rpad(k), uniform_top(rinfo[k & 1]), 0, LF, m);
+    clip_words<NPL>(m, WL);
+    const int sg = sa ^ (__any_sync(kFull, rinfo[2 + (k & 1)]) ? 1 : 0);
     if (omag) {
-#pragma unroll
-      for (int c = 0; c < NPL; c++)
-        if (lane + 32 * c < WL) omag[lane + 32 * c] = m[c];
-    }
-    if (otop) {
+      reg_store<NPL>(omag, m, WL);
       const int tp = warp_top<NPL>(m, WL);
-      if (lane == 0) *otop = (uint8_t)tp;
+      if (lane == 0) {
+        *otop = (uint8_t)tp;
+        *osign = (uint8_t)sg;
+      }
     }
-    if (osign && lane == 0) *osign = (uint8_t)sg;
-    if (sg) warp_negate<NPL>(m, WL);
+    u32 v[NPL];
 #pragma unroll
-    for (int c = 0; c < NPL; c++)
-      if (lane + 32 * c < WL) out[lane + 32 * c] = m[c];
+    for (int c = 0; c < NPL; c++) v[c] = m[c];
+    if (sg) warp_negate<NPL>(v, WL);
+    reg_store<NPL>(out, v, WL);
     __syncwarp();
   };
+  // the scratch operands start as zeros: the pads, and the words from WL on, stay so
+  for (int e = tid; e < (int)(kWarpsS * sizeof(WarpScratchT<NPL>) / 4); e += kThreadsS) reinterpret_cast<u32*>(ws)[e] = 0u;
+  for (int e = tid; e < 4 * NWD + 4 + 4 * kPadWords<NPL>; e += kThreadsS) nw[e] = 0u;
+  __syncthreads();
   // pivot 0 reads a_00 from the tile itself while warps 1.. copy the triangle into shared memory
-  if (warp == 0) pivot(0, GLOBAL ? ent(0, 0) : G);
-  else if (!GLOBAL)
+  u32 D[NPL], m0[NPL];
+  if (warp == 0) {
+    reg_load<NPL>(GLOBAL ? ent(0, 0) : G, D, WL);
+    pivot(0, D);
+  } else if (!GLOBAL) {
     for (int i = warp - 1; i < BT; i += kWarpsS - 1) copy_row(i, true);
+  }
   __syncthreads();
   // Step k: column k scaled by r_k; then, with one pivot of look-ahead, warp 0 updates a_{k+1,k+1} and runs
   // pivot k+1's Newton chain while warps 1.. apply the rest of step k's trailing update.  Every entry gets
@@ -877,27 +998,34 @@ __global__ void __launch_bounds__(kThreadsS) chol_tiles_k(u32* __restrict__ A, u
     if (warp == 0) {
       if (k + 1 < BT) {
         u32* aik = ent(k + 1, k);
-        mul_r(aik, k, aik, colmag + (size_t)(k + 1) * WP, colsign + k + 1, coltop + k + 1);
+        mul_r(aik, k, aik, colmag + (size_t)(k + 1) * WP, colsign + k + 1, coltop + k + 1, m0);
       }
       asm volatile("bar.arrive 1, %0;" ::"r"(kThreadsS) : "memory");
     } else {
       if (warp == kWarpsS - 1) {
         u32* akk = ent(k, k);
-        mul_r(akk, k, akk, nullptr, nullptr, nullptr);
+        mul_r(akk, k, akk, nullptr, nullptr, nullptr, m0);
       }
       for (int i = k + 1 + warp; i < BT; i += kWarpsS - 1) {
         u32* aik = ent(i, k);
-        mul_r(aik, k, aik, colmag + (size_t)i * WP, colsign + i, coltop + i);
+        mul_r(aik, k, aik, colmag + (size_t)i * WP, colsign + i, coltop + i, m0);
       }
       asm volatile("bar.sync 1, %0;" ::"r"(kThreadsS) : "memory");
     }
     if (k == BT - 1) break;
     if (warp == 0) {
       u32* dn = ent(k + 1, k + 1);                // a_{k+1,k+1} -= l_{k+1,k}^2 (a square of magnitudes)
-      const u32* lk = colmag + (size_t)(k + 1) * WP;
-      wmul_core<NPL, true>(lk, coltop[k + 1], lk, coltop[k + 1], 0, WL, LF, st1);
-      warp_addsub<NPL>(dn, dn, st1, true, WL);
-      pivot(k + 1, dn);
+      const int tl = warp_top<NPL>(m0, WL);
+      reg_store_from<NPL>(rm, m0, 0);
+      __syncwarp();
+      u32 sq[NPL];
+      wmul_pad<NPL>(rm, tl, 0, rm, tl, 0, LF, sq);
+      clip_words<NPL>(sq, WL);
+      reg_load<NPL>(dn, D, WL);
+      reg_addsub<NPL>(D, D, sq, true, WL);
+      reg_store<NPL>(dn, D, WL);
+      __syncwarp();
+      pivot(k + 1, D);
     } else {
       const int m = BT - k - 1, npairs = m * (m + 1) / 2;
       for (int p = 1 + tid - 32; p < npairs; p += kThreadsS - 32) {   // a_ij -= l_ik l_jk, k < j <= i, but (k+1, k+1)
@@ -936,11 +1064,12 @@ __global__ void __launch_bounds__(kThreadsS) trinv_tiles_k(const u32* __restrict
   const int WP = pitch(WL);
   u32* Xm = GLOBAL ? S + (size_t)blockIdx.x * 528 * WP : sm;     // slots tri(i, k), lower triangle
   // |l_ij| of column j by row i in Lcol + (j & 1) 32 WP (column j + 1 is read from the tile during step j's
-  // products and stored after them); the pivot reciprocals r_i in RIs
+  // products and stored after them); |r_i| in the padded operand rpad(i) while row i is finished
   u32* Lcol = GLOBAL ? sm : sm + 528 * WP;
-  u32* RIs = Lcol + 64 * WP;
-  WarpScratchT<NPL>* ws = reinterpret_cast<WarpScratchT<NPL>*>(RIs + 32 * WP);
-  uint8_t* xs = reinterpret_cast<uint8_t*>(ws + kWarpsS);             // signs, tops of finished x
+  WarpScratchT<NPL>* ws = reinterpret_cast<WarpScratchT<NPL>*>(((uintptr_t)(Lcol + 64 * WP) + 15) & ~(uintptr_t)15);
+  u32* pads = reinterpret_cast<u32*>(ws + kWarpsS);
+  auto rpad = [&](int i) { return pads + (i & 1) * kPadWords<NPL> + kPadLo<NPL>; };
+  uint8_t* xs = reinterpret_cast<uint8_t*>(pads + 2 * kPadWords<NPL>);   // signs, tops of finished x
   uint8_t* xt = xs + 528;
   uint8_t* ls = xt + 528;                                        // signs, tops of the columns of L (2 x 32)
   uint8_t* lt = ls + 64;
@@ -949,12 +1078,13 @@ __global__ void __launch_bounds__(kThreadsS) trinv_tiles_k(const u32* __restrict
   const u32* RI = RINV + (size_t)blockIdx.x * BT * WL;
   u32* XG = X + (size_t)blockIdx.x * BT * BT * WL;
   for (int e = tid; e < 528 * WP; e += kThreadsS) Xm[e] = 0;
-  for (int i = warp; i < BT; i += kWarpsS)
-    for (int w = lane; w < WL; w += 32) RIs[i * WP + w] = RI[(size_t)i * WL + w];
+  // scratch operands start as zeros: the pads, and the words from WL on, stay so
+  for (int e = tid; e < (int)(kWarpsS * sizeof(WarpScratchT<NPL>) / 4) + 2 * kPadWords<NPL>; e += kThreadsS)
+    reinterpret_cast<u32*>(ws)[e] = 0u;
   __syncthreads();
   for (int i = warp; i < BT; i += kWarpsS) {                     // x_ii = r_i
     int top;
-    const int sg = load_mag<NPL>(RIs + i * WP, Xm + (size_t)tri(i, i) * WP, WL, top);
+    const int sg = load_mag<NPL>(RI + (size_t)i * WL, Xm + (size_t)tri(i, i) * WP, WL, top);
     if (lane == 0) {
       xs[tri(i, i)] = (uint8_t)sg;
       xt[tri(i, i)] = (uint8_t)top;
@@ -969,6 +1099,12 @@ __global__ void __launch_bounds__(kThreadsS) trinv_tiles_k(const u32* __restrict
     }
   }
   __syncthreads();
+  auto fill_rpad = [&](int i) {                                  // one warp
+    u32 v[NPL];
+    reg_load<NPL>(Xm + (size_t)tri(i, i) * WP, v, WL);
+    reg_store_from<NPL>(rpad(i), v, 0);
+  };
+  if (warp == kWarpsS - 1) fill_rpad(1);
   for (int j = 0; j < BT - 1; j++) {
     const u32* Lc = Lcol + (j & 1) * 32 * WP;
     const uint8_t *lsj = ls + (j & 1) * 32, *ltj = lt + (j & 1) * 32;
@@ -1001,18 +1137,29 @@ __global__ void __launch_bounds__(kThreadsS) trinv_tiles_k(const u32* __restrict
     __syncthreads();
     for (int k = warp; k <= j; k += kWarpsS) {                   // x_{j+1,k} = -(sum) r_{j+1}
       const int ei = tri(j + 1, k);
-      wmul<NPL>(Xm + (size_t)ei * WP, RIs + (j + 1) * WP, 0, WL, LF, ws[warp], nullptr, Xm + (size_t)ei * WP,
-           xs + ei, xt + ei);
-      if (lane == 0) xs[ei] ^= 1;                                // the negation
+      WarpScratchT<NPL>& sc = ws[warp];
+      u32 m[NPL];
+      int ta;
+      const int sa = load_mag<NPL>(Xm + (size_t)ei * WP, sc.xa, WL, ta);
+      __syncwarp();
+      wmul_pad<NPL>(sc.xa, ta, 0, rpad(j + 1), uniform_top(xt[tri(j + 1, j + 1)]), 0, LF, m);
+      clip_words<NPL>(m, WL);
+      reg_store<NPL>(Xm + (size_t)ei * WP, m, WL);
+      const int top = warp_top<NPL>(m, WL);
+      if (lane == 0) {
+        xt[ei] = (uint8_t)top;
+        xs[ei] = (uint8_t)(sa ^ xs[tri(j + 1, j + 1)] ^ 1);      // the negation
+      }
       __syncwarp();
     }
+    if (warp == kWarpsS - 1 && j + 2 < BT) fill_rpad(j + 2);     // row j + 2's, in the buffer that row j used
     {
       u32* Ln = Lcol + ((j + 1) & 1) * 32 * WP;                  // column j + 1 as magnitudes
 #pragma unroll
       for (int q = 0; q < 2; q++) {
         const int i = j + 2 + warp + q * kWarpsS;
         if (i < BT) {
-          const int sg = (int)(reg_word<NPL>(pf[q], WL - 1) >> 31);
+          const int sg = reg_sign<NPL>(pf[q], WL) ? 1 : 0;
           if (sg) warp_negate<NPL>(pf[q], WL);
           const int top = warp_top<NPL>(pf[q], WL);
           reg_store<NPL>(Ln + (size_t)i * WP, pf[q], WL);
