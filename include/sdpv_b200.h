@@ -112,12 +112,17 @@ int sdpv_tune_get(int knob, int* value);
  * Record: byte is_zero; unless zero, int32 size, int64 exp, nl 64-bit limbs; value = sign(size) M
  * 2^(64 (exp - |size|)).  Replaces decode_bigfloats / encode_bigfloats (sdpvibe/_bigfloat.c:16-111).
  * sdpv_bigfloat_index (host, no launch): offsets of n records from pos; SDPV_EINVAL if truncated/corrupt.
- * sdpv_bigfloat_unpack: device records at offsets -> planar (L, n) limbs + exponents, mantissa rounded half
- *   up to at most 32 L - 2 bits (L <= 64, nl <= 64).
+ * sdpv_bigfloat_load: the records from host byte pos copied to dbuf (dbytes >= min(len - pos, n (13 + 8 nl)))
+ *   while a host pass finds their offsets (offsets: n host words, relative to pos) and *end; *regular = 1 when no
+ *   record is a zero record, else the offsets are copied to doffsets too.  SDPV_EINVAL if truncated/corrupt.
+ * sdpv_bigfloat_unpack: device records at offsets (NULL: every record 13 + 8 nl bytes) -> planar (L, n) limbs +
+ *   exponents, mantissa rounded half up to at most 32 L - 2 bits (L <= 64, nl <= 64).
  * sdpv_bigfloat_pack: planar limbs + exponents -> device records at offsets (1 or 13 + 8 nl bytes each);
  *   a mantissa wider than nl limbs sets SDPV_ERRBIT_OVERFLOW. */
 int sdpv_bigfloat_index(const uint8_t* buf, int64_t len, int64_t pos, int64_t n, int nl, int64_t* offsets,
                         int64_t* end);
+int sdpv_bigfloat_load(const uint8_t* buf, int64_t len, int64_t pos, int64_t n, int nl, uint8_t* dbuf, int64_t dbytes,
+                       int64_t* offsets, int64_t* doffsets, int* regular, int64_t* end, void* stream);
 int sdpv_bigfloat_unpack(const uint8_t* buf, const int64_t* offsets, int64_t n, int nl, int L, int32_t* out,
                          int64_t* exps, void* stream);
 int sdpv_bigfloat_pack(const int32_t* m, const int64_t* e, int64_t n, int L, int nl, const int64_t* offsets,

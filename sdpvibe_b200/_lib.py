@@ -41,6 +41,7 @@ _SIGS = {
     "sdpv_mpf_from_f64": [_I, _L, _P, _P, _P, _P],
     "sdpv_schur_assemble": [_I, _L, _I, _I, _I, _P, _P, _P, _P, _P, _P, _L, _P, _P, _P],
     "sdpv_bigfloat_index": [_P, _L, _L, _L, _I, _P, _P],
+    "sdpv_bigfloat_load": [_P, _L, _L, _L, _I, _P, _L, _P, _P, ctypes.POINTER(_I), ctypes.POINTER(_L), _P],
     "sdpv_tune_set": [_I, _I],
     "sdpv_tune_get": [_I, _P],
     "sdpv_bigfloat_unpack": [_P, _P, _L, _I, _I, _P, _P, _P],

@@ -2,9 +2,9 @@
 read and written with the number records decoded and encoded on the GPU (drop-in for the binary paths of
 ``sdpvibe.sdp_io``, sdpvibe/sdp_io.py:143-297, and its C codec sdpvibe/_bigfloat.c).
 
-  decode_bigfloats(buf, pos, n, nl, L) -> (MPF (n,) on the device, end position): offsets of the records
-      from one pass over their zero flags on the host (sdpv_bigfloat_index), the bytes copied once, one GPU
-      thread per record (sdpv_bigfloat_unpack) straight into limb planes
+  decode_bigfloats(buf, pos, n, nl, L) -> (MPF (n,) on the device, end position): the bytes copied straight from
+      the caller's buffer while one host pass over the zero flags gives the records' offsets
+      (sdpv_bigfloat_load), one GPU thread per record (sdpv_bigfloat_unpack) straight into limb planes
   encode_bigfloats(A, nl) -> bytes (sdpv_bigfloat_pack)
   BinReader(buf, L): the archive (header, El::Matrix<BigFloat> column-major with a leading dimension,
       std::vector<BigFloat>) with matrices and vectors as device MPFs
@@ -39,18 +39,20 @@ def decode_bigfloats(buf, pos, n, nl, L):
         return MPF(torch.zeros((L, 0), dtype=torch.int32, device=dev),
                    torch.zeros((0,), dtype=torch.int64, device=dev)), pos
     offs = np.empty(n, dtype=np.int64)
-    end = ctypes.c_int64(0)
-    st = _lib.lib().sdpv_bigfloat_index(arr.ctypes.data_as(ctypes.c_void_p), len(arr), pos, n, nl,
-                                        offs.ctypes.data_as(ctypes.c_void_p), ctypes.addressof(end))
-    if st != _lib.OK:
-        raise ValueError("truncated or corrupt binary block data")
-    lo, hi = int(offs[0]), int(end.value)
-    dbuf = torch.from_numpy(np.array(arr[lo:hi])).to(dev)           # one copy of the records, then H2D
-    doffs = torch.from_numpy(offs - lo).to(dev)
+    end, regular = ctypes.c_int64(0), ctypes.c_int(0)
+    size = max(0, min(len(arr) - pos, n * (13 + 8 * nl)))
+    dbuf = torch.empty((size,), dtype=torch.uint8, device=dev)
+    doffs = torch.empty((n,), dtype=torch.int64, device=dev)
     m = torch.empty((L, n), dtype=torch.int32, device=dev)
     e = torch.empty((n,), dtype=torch.int64, device=dev)
-    _lib.call("sdpv_bigfloat_unpack", _lib.ptr(dbuf), _lib.ptr(doffs), n, nl, L, _lib.ptr(m), _lib.ptr(e), _lib.stream())
-    return MPF(m, e), hi
+    st = _lib.lib().sdpv_bigfloat_load(arr.ctypes.data, len(arr), pos, n, nl, dbuf.data_ptr(), size, offs.ctypes.data,
+                                       doffs.data_ptr(), ctypes.byref(regular), ctypes.byref(end), _lib.stream())
+    if st == _lib.EINVAL:
+        raise ValueError("truncated or corrupt binary block data")
+    _lib.check(st, "sdpv_bigfloat_load")
+    _lib.call("sdpv_bigfloat_unpack", dbuf.data_ptr(), None if regular.value else doffs.data_ptr(), n, nl, L, _lib.ptr(m),
+              _lib.ptr(e), _lib.stream())
+    return MPF(m, e), int(end.value)
 
 
 def encode_bigfloats(A, nl):

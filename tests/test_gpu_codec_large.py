@@ -1,0 +1,38 @@
+"""Reading binary records on both sides of the size (1 MiB) from which the flag pass runs on its own thread: all
+records of full length (no offsets uploaded) or zeros among them, at an offset into a longer buffer, truncated
+and corrupt ones; against the encoder's input."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 5000, 9000])
+@pytest.mark.parametrize("zeros", [False, True])
+def test_round_trip(n, zeros):
+    from sdpvibe_b200 import mpf
+    from sdpvibe_b200.sdp_io import decode_bigfloats, encode_bigfloats
+    L, nl = 26, 18
+    g = torch.Generator(device="cuda").manual_seed(n)
+    w = torch.randint(-(1 << 31), (1 << 31) - 1, (L, n), dtype=torch.int32, device="cuda", generator=g)
+    A = mpf.normalize(w, torch.randint(-900, 900, (n,), device="cuda", generator=g), L)
+    if zeros:
+        A.m[:, ::3] = 0
+        A.e[::3] = mpf.EZ
+    rec = encode_bigfloats(A, nl)
+    buf = b"\x07" * 11 + rec + b"tail"
+    B, end = decode_bigfloats(buf, 11, n, nl, L)
+    assert end == 11 + len(rec)
+    C = mpf.normalize(B.m, B.e, L)                                   # decoded mantissas are not renormalised
+    assert torch.equal(C.m, A.m) and torch.equal(C.e, A.e)
+    with pytest.raises(ValueError):                                  # one record short
+        decode_bigfloats(buf[:11 + len(rec) - 1], 11, n, nl, L)
+    with pytest.raises(ValueError):
+        decode_bigfloats(buf, len(buf) + 3, n, nl, L)
+    bad = bytearray(buf)
+    last = len(bad) - 4 - (1 if zeros and (n - 1) % 3 == 0 else 13 + 8 * nl)
+    if bad[last] == 0:
+        bad[last + 1:last + 5] = (nl + 1).to_bytes(4, "little")      # |size| > nl in the last record
+        with pytest.raises(ValueError):
+            decode_bigfloats(bytes(bad), 11, n, nl, L)
