@@ -512,7 +512,7 @@ CS_BLOCKS, CS_NMIN, CS_NMAX, CS_NRHS, CS_L = 600, 8, 160, 8, 26
 TRACE_NAMES = ("sdpv_chol_tiles", "sdpv_trinv_tiles", "sdpv_residues", "sdpv_residues_u8", "sdpv_residues_rows",
                "sdpv_rns_gemm", "sdpv_rns_gemm_grouped", "sdpv_crt_norm", "sdpv_crt_block", "sdpv_shift_round",
                "sdpv_add_same", "sdpv_bitlen", "sdpv_badd_align", "sdpv_mpf_norm", "sdpv_mpf_mul", "sdpv_mpf_add",
-               "sdpv_top_max", "sdpv_gemm_operands", "sdpv_align", "sdpv_align_t", "sdpv_align_rows", "sdpv_grp_copy", "sdpv_grp_finish_fixed",
+               "sdpv_top_max", "sdpv_gemm_operands", "sdpv_gemm_exponents", "sdpv_gemm_tall", "sdpv_align", "sdpv_align_t", "sdpv_align_rows", "sdpv_grp_copy", "sdpv_grp_finish_fixed",
                "sdpv_grp_solve_round", "sdpv_grp_merge", "sdpv_grp_tile_widen",
                "sdpv_grp_tile_narrow")
 

@@ -170,6 +170,18 @@ int sdpv_align_t(const int32_t* m, const int64_t* e, int L, int64_t nb, int64_t 
 int sdpv_gemm_operands(const int32_t* Am, const int64_t* Ae, const int32_t* Bm, const int64_t* Be, int L, int64_t nb,
                        int64_t M, int64_t K, int64_t N, int transA, int transB, int64_t ld, int32_t* X, int64_t* Ea,
                        int64_t* Eb, int64_t ldE, void* stream);
+/* The exponents alone, as sdpv_gemm_operands makes them. */
+int sdpv_gemm_exponents(const int32_t* Am, const int64_t* Ae, const int32_t* Bm, const int64_t* Be, int L, int64_t nb,
+                        int64_t M, int64_t K, int64_t N, int transA, int transB, int64_t* Ea, int64_t* Eb, int64_t ldE,
+                        void* stream);
+/* C (M, N) = A^T op(B) for A stored (K, M), N <= 4 columns of op(B) (stored (K, N), or (N, K) when transB), L <= 32,
+ * K <= 65536, without residues: the entries' digits against Toeplitz operands of the columns on the tensor cores
+ * (see matvec.cu), rounded once as mpf.gemm.  Ea (M) and Eb (N) from sdpv_gemm_exponents; ws: device workspace of
+ * sdpv_gemm_tall_workspace bytes (0: shape not taken), 256-byte aligned. */
+int sdpv_gemm_tall_workspace(int L, int64_t M, int64_t K, int64_t N, int64_t* bytes);
+int sdpv_gemm_tall(const int32_t* Am, const int64_t* Ae, const int32_t* Bm, const int64_t* Be, int L, int64_t M, int64_t K,
+                   int64_t N, int transB, const int64_t* Ea, const int64_t* Eb, void* ws, int64_t ws_bytes, int32_t* O,
+                   int64_t* eO, void* stream);
 /* The transposed alignment written as operand rows for sdpv_residues_rows: entry (b, r, c) of m becomes row
  * (b C + c) Rp + r of out (nb, C, Rp, rb) uint8, rb = 128 bytes for Lout <= 31, 256 for Lout <= 63: the Lout
  * aligned limbs little endian, then a sign byte (1 when the result is negative) at byte 4 Lout, then zeros;

@@ -48,6 +48,9 @@ _SIGS = {
     "sdpv_bigfloat_pack": [_P, _P, _L, _I, _I, _P, _P, _P],
     "sdpv_top_max": [_P, _P, _I, _L, _L, _L, _I, _P, _P],
     "sdpv_gemm_operands": [_P, _P, _P, _P, _I, _L, _L, _L, _L, _I, _I, _L, _P, _P, _P, _L, _P],
+    "sdpv_gemm_exponents": [_P, _P, _P, _P, _I, _L, _L, _L, _L, _I, _I, _P, _P, _L, _P],
+    "sdpv_gemm_tall_workspace": [_I, _L, _L, _L, ctypes.POINTER(_L)],
+    "sdpv_gemm_tall": [_P, _P, _P, _P, _I, _L, _L, _L, _I, _P, _P, _P, _L, _P, _P, _P],
     "sdpv_align": [_P, _P, _I, _L, _L, _L, _P, _I, _I, _I, _P, _P],
     "sdpv_residues": [_P, _P, _L, _L, _L, _L, _I, _I, _P, _P, _L, _P],
     "sdpv_residues_u8": [_P, _P, _L, _L, _L, _L, _I, _I, _P, _P, _L, _P],

@@ -599,6 +599,50 @@ extern "C" int sdpv_align_t(const int32_t* m, const int64_t* e, int L, int64_t n
   return sdpv::launch_status();
 }
 
+namespace {
+// The operands of C = op(A) op(B); a single column is contiguous and read as a row.
+void operand_sides(const int32_t* Am, const int64_t* Ae, const int32_t* Bm, const int64_t* Be, int64_t nb, int64_t M,
+                   int64_t K, int64_t N, int transA, int transB, int64_t* Ea, int64_t* Eb, int64_t ldE, OpSide& A,
+                   OpSide& B) {
+  A = OpSide{Am, Ae, nb, transA ? K : M, transA ? M : K, transA && M > 1, Ea, M, 0, 0, 1};
+  B = OpSide{Bm, Be, nb, transB ? N : K, transB ? K : N, !transB && N > 1, Eb, ldE, nb * M, 0, 1};
+  if (transA && M == 1) A.R = 1, A.C = K;
+  if (!transB && N == 1) B.R = 1, B.C = K;
+}
+
+// The exponents of both sides (Ea, Eb).
+int operand_exponents(OpSide A, OpSide B, int L, cudaStream_t st) {
+  for (OpSide* S : {&A, &B}) {
+    if (S->strided) {
+      S->split = (int)((S->R + kTopRows - 1) / kTopRows);
+      S->blocks = S->nb * ((S->C + 31) / 32) * S->split;
+    } else {
+      S->blocks = S->C > kWarpVec ? S->nb * S->R : (S->nb * S->R + 7) / 8;
+    }
+    // tops of split columns meet by atomic maximum: start below every top (0x80 bytes are below EZ)
+    if (S->split > 1) {
+      const size_t count = (size_t)((S->nb - 1) * S->ldE + S->per());
+      cudaError_t ce = cudaMemsetAsync(S->E, 0x80, count * 8, st);
+      if (ce != cudaSuccess) return sdpv::set_cuda_error(ce);
+    }
+  }
+  if (A.blocks + B.blocks > 0x7fffffff) return SDPV_EINVAL;
+  gemm_tops_kernel<<<(unsigned)(A.blocks + B.blocks), kThreads, 0, st>>>(A, B, L);
+  for (OpSide* S : {&A, &B})
+    if (S->split > 1) gemm_exps_kernel<<<blocks(S->nb * S->per()), kThreads, 0, st>>>(*S, L);
+  return sdpv::launch_status();
+}
+}  // namespace
+
+extern "C" int sdpv_gemm_exponents(const int32_t* Am, const int64_t* Ae, const int32_t* Bm, const int64_t* Be, int L,
+                                   int64_t nb, int64_t M, int64_t K, int64_t N, int transA, int transB, int64_t* Ea,
+                                   int64_t* Eb, int64_t ldE, void* stream) {
+  if (L < 1 || L > 160 || nb < 1 || M < 1 || K < 1 || N < 1 || ldE < N || nb > 65535) return SDPV_EINVAL;
+  OpSide A, B;
+  operand_sides(Am, Ae, Bm, Be, nb, M, K, N, transA, transB, Ea, Eb, ldE, A, B);
+  return operand_exponents(A, B, L, sdpv::as_stream(stream));
+}
+
 // Both operands of C = op(A) op(B), aligned and stacked: X (L, nb M + nb N, ld) holds the nb M rows of op(A),
 // then the nb N columns of op(B), K entries each; Ea (nb M) and Eb (nb rows of ldE) their exponents.
 extern "C" int sdpv_gemm_operands(const int32_t* Am, const int64_t* Ae, const int32_t* Bm, const int64_t* Be, int L,
@@ -606,34 +650,10 @@ extern "C" int sdpv_gemm_operands(const int32_t* Am, const int64_t* Ae, const in
                                   int32_t* X, int64_t* Ea, int64_t* Eb, int64_t ldE, void* stream) {
   if (L < 1 || L > 64 || nb < 1 || M < 1 || K < 1 || N < 1 || ld < K || ldE < N || nb > 65535) return SDPV_EINVAL;
   cudaStream_t st = sdpv::as_stream(stream);
-  // a single column is contiguous: it is read as a row
-  OpSide A{Am, Ae, nb, transA ? K : M, transA ? M : K, transA && M > 1, Ea, M, 0, 0, 1};
-  OpSide B{Bm, Be, nb, transB ? N : K, transB ? K : N, !transB && N > 1, Eb, ldE, nb * M, 0, 1};
-  if (transA && M == 1) A.R = 1, A.C = K;
-  if (!transB && N == 1) B.R = 1, B.C = K;
-  bool raw = false;
-  for (OpSide* S : {&A, &B}) {
-    if (S->strided) {
-      S->split = (int)((S->R + kTopRows - 1) / kTopRows);
-      S->blocks = S->nb * ((S->C + 31) / 32) * S->split;
-      raw = raw || S->split > 1;
-    } else {
-      S->blocks = S->C > kWarpVec ? S->nb * S->R : (S->nb * S->R + 7) / 8;
-    }
-  }
-  if (A.blocks + B.blocks > 0x7fffffff) return SDPV_EINVAL;
-  if (raw) {
-    // tops of split columns meet by atomic maximum: start below every top (0x80 bytes are below EZ)
-    for (OpSide* S : {&A, &B})
-      if (S->split > 1) {
-        const size_t count = (size_t)((S->nb - 1) * S->ldE + S->per());
-        cudaError_t ce = cudaMemsetAsync(S->E, 0x80, count * 8, st);
-        if (ce != cudaSuccess) return sdpv::set_cuda_error(ce);
-      }
-  }
-  gemm_tops_kernel<<<(unsigned)(A.blocks + B.blocks), kThreads, 0, st>>>(A, B, L);
-  for (OpSide* S : {&A, &B})
-    if (S->split > 1) gemm_exps_kernel<<<blocks(S->nb * S->per()), kThreads, 0, st>>>(*S, L);
+  OpSide A, B;
+  operand_sides(Am, Ae, Bm, Be, nb, M, K, N, transA, transB, Ea, Eb, ldE, A, B);
+  const int rc = operand_exponents(A, B, L, st);
+  if (rc != SDPV_OK) return rc;
   for (OpSide* S : {&A, &B})
     S->blocks = S->strided ? S->nb * ((S->C + TC - 1) / TC) * ((S->R + ATR - 1) / ATR)
                            : (S->nb * S->R * S->C + kThreads - 1) / kThreads;

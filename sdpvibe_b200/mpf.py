@@ -8,6 +8,7 @@ Elementwise operations are libsdpv_b200 kernels with the reference's rounding (m
 renormalises each entry inside the CRT kernel (one launch for CRT + rounding).  ``GramAcc`` keeps
 Q = sum_c P_c^T P_c in residue form across chunks (lower-triangle tiles only) with one CRT at the end.
 """
+import ctypes
 import os
 
 import mpmath as mp
@@ -378,6 +379,34 @@ def _align_rows(A):
     return out.view(A.m.shape), E.view(A.shape[:-1])
 
 
+# Entries of A from which one or two columns are multiplied without residues (_gemm_tall; three or four, two passes
+# over A: from four times as many).  Measured at L = 26, without / through residues: 200 x 1000 by one column 59 /
+# 85 us, 2000 x 128 99 / 102, 256 x 256 58 / 53; by three 1000 x 1000 230 / 244, 600 x 600 165 / 130.
+TALL_MIN = 1 << 17
+
+
+def _gemm_tall(A, B, L, M, K, N, transB):
+    """C (M, N) = A^T op(B) with few columns: A's digits against the columns' Toeplitz operands (sdpv_gemm_tall),
+    every entry of A read once and never written back; None where the kernel does not take the shape."""
+    need = ctypes.c_int64()
+    _lib.check(_lib.lib().sdpv_gemm_tall_workspace(L, M, K, N, ctypes.byref(need)), "sdpv_gemm_tall_workspace")
+    if not need.value:
+        return None
+    E = torch.empty((M + N,), dtype=torch.int64, device=dev)
+    ws = torch.empty((need.value,), dtype=torch.uint8, device=dev)
+    Om = torch.empty((L, M, N), dtype=torch.int32, device=dev)
+    Oe = torch.empty((M, N), dtype=torch.int64, device=dev)
+    ops = [t.contiguous() for t in (A.m, A.e, B.m, B.e)]
+    ptrs = [_lib.ptr(t) for t in ops]
+    ea = E.data_ptr()
+    eb = ea + 8 * M
+    st = _lib.stream()
+    _lib.call("sdpv_gemm_exponents", *ptrs, L, 1, M, K, N, 1, int(transB), ea, eb, N, st)
+    _lib.call("sdpv_gemm_tall", *ptrs, L, M, K, N, int(transB), ea, eb, ws.data_ptr(), need.value, Om.data_ptr(),
+              Oe.data_ptr(), st)
+    return MPF(Om, Oe)
+
+
 def gemm(A, B, transA=False, transB=False):
     """C = op(A) op(B) (2-d, or batched 3-d (nb, ., .)); exact products, every entry rounded once
     (operands aligned per row of op(A) / column of op(B)) (sdpvibe/mpf.py:401-452)."""
@@ -392,6 +421,10 @@ def gemm(A, B, transA=False, transB=False):
     shape = (nb, M, N) if len(sa) == 3 else (M, N)
     if not (nb and M and N and K):
         return zeros(shape, L)                                      # no entries, or empty sums
+    if transA and nb == 1 and N <= 4 and M * K >= TALL_MIN * (1 if N <= 2 else 4):
+        C = _gemm_tall(A, B, L, M, K, N, transB)
+        if C is not None:
+            return C.reshape(*shape)
     # op(A) rows and op(B) columns aligned to their own exponents, the transposes fused into the alignment, both
     # stacked in one operand buffer (rows padded to 16 bytes for the decomposition's bulk copies)
     ld = (K + 3) & ~3
