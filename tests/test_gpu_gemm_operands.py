@@ -8,7 +8,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(1, 1, 1, 1), (1, 5, 512, 3), (1, 3, 513, 2), (1, 33, 1100, 31), (3, 9, 41, 1), (2, 1, 600, 40),
+SHAPES = [(1, 1, 1, 1), (5, 7, 64, 9), (5, 7, 65, 9), (1, 5, 512, 3), (1, 3, 513, 2), (1, 33, 1100, 31), (3, 9, 41, 1), (2, 1, 600, 40),
           (4, 21, 44, 17), (1, 1, 1030, 1), (2, 40, 7, 65)]
 
 
