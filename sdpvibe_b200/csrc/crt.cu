@@ -50,6 +50,36 @@ __device__ __forceinline__ u64 digit_word(const u32* z) {
   return (u64)(z[1] * 256u + z[0]) + (u64)(z[3] * 256u + z[2]) * 65536ull;
 }
 
+// Residues v[q] of moduli gb + q -> y = residue inv mod m in [0, m), its digits into the entry's rows of Y.
+__device__ __forceinline__ void store_digits(const CrtMod* TB, int gb, const int (&v)[32], int row, uint8_t* Yh,
+                                             uint8_t* Yl) {
+#pragma unroll
+  for (int h = 0; h < 2; h++) {                        // 16 moduli per 16-byte chunk
+    u32 ph[4], pl[4];
+#pragma unroll
+    for (int q4 = 0; q4 < 4; q4++) {
+      u32 y[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int a = v[16 * h + 4 * q4 + u];
+        const int4 c = *reinterpret_cast<const int4*>(&TB[gb + 16 * h + 4 * q4 + u]);
+        // x = a inv, q = round(x / m) from the float product (off by less than 0.002): |x - q m| <= 0.502 m, so one
+        // correction gives y in [0, m)
+        const float fa = __int_as_float(0x4B008000 + a) - 8421376.0f;
+        const int qb = __float_as_int(fmaf(fa, __int_as_float(c.z), 12582912.0f));
+        const int x = a * c.y + c.w - qb * c.x;
+        y[u] = (u32)(x + ((x >> 31) & c.x));
+      }
+      const u32 p01 = y[0] + (y[1] << 16), p23 = y[2] + (y[3] << 16);
+      ph[q4] = __byte_perm(p01 >> 7, p23 >> 7, 0x6420);
+      pl[q4] = __byte_perm(p01, p23, 0x6420) & 0x7F7F7F7Fu;
+    }
+    const int g16 = gb + 16 * h, kt = g16 >> 7, chunk = (g16 & 127) >> 4;
+    *reinterpret_cast<uint4*>(Yh + kt * kSlice + sw128_off(row, chunk)) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
+    *reinterpret_cast<uint4*>(Yl + kt * kSlice + sw128_off(row, chunk)) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+  }
+}
+
 // Dynamic shared memory: [head] [Y: 2 ktc slices] [nslot chunk slots of 2 ktc slices].  The whole table stays
 // resident where it fits (n <= 128); else its chunks pass through the slots, from L2, once per tile.
 template <int MODE, bool WIDE>
@@ -117,33 +147,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 
   while (true) {
     // ---- pre-pass: the digits of y_i
-    auto digits = [&](int gb, const int (&v)[32]) {
-#pragma unroll
-      for (int h = 0; h < 2; h++) {                    // 16 moduli per 16-byte chunk
-        u32 ph[4], pl[4];
-#pragma unroll
-        for (int q4 = 0; q4 < 4; q4++) {
-          u32 y[4];
-#pragma unroll
-          for (int u = 0; u < 4; u++) {
-            const int a = v[16 * h + 4 * q4 + u];
-            const int4 c = *reinterpret_cast<const int4*>(&TB[gb + 16 * h + 4 * q4 + u]);
-            // x = a inv, q = round(x / m) from the float product (off by less than 0.002): |x - q m| <= 0.502 m,
-            // so one correction gives y in [0, m)
-            const float fa = __int_as_float(0x4B008000 + a) - 8421376.0f;
-            const int qb = __float_as_int(fmaf(fa, __int_as_float(c.z), 12582912.0f));
-            const int x = a * c.y + c.w - qb * c.x;
-            y[u] = (u32)(x + ((x >> 31) & c.x));
-          }
-          const u32 p01 = y[0] + (y[1] << 16), p23 = y[2] + (y[3] << 16);
-          ph[q4] = __byte_perm(p01 >> 7, p23 >> 7, 0x6420);
-          pl[q4] = __byte_perm(p01, p23, 0x6420) & 0x7F7F7F7Fu;
-        }
-        const int g16 = gb + 16 * h, kt = g16 >> 7, chunk = (g16 & 127) >> 4;
-        *reinterpret_cast<uint4*>(Yh + kt * kSlice + sw128_off(tid, chunk)) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
-        *reinterpret_cast<uint4*>(Yl + kt * kSlice + sw128_off(tid, chunk)) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
-      }
-    };
+    auto digits = [&](int gb, const int (&v)[32]) { store_digits(TB, gb, v, tid, Yh, Yl); };
     for (int gb = 0; gb < n; gb += 64) {
       if (gb + 32 < n) load(gb + 32, vb);
       digits(gb, va);
@@ -262,6 +266,192 @@ __global__ void __launch_bounds__(kThreads, 2)
   if (warp == 0) tmem_dealloc(tmem, tcols);
 }
 
+// The same for calls of many tiles with n <= 128 (one or two digit chunks): kWide tiles at a time on an SM, each worked
+// by its own four warps, which share one copy of the table.  TMEM then holds one chunk per tile, so the chunks run
+// one after the other, the first one's words waiting in registers while the second's product still reads Y.
+// Measured against two one-tile CTAs per SM (8 warps, latency-bound): 158760 entries at 116 moduli 68 -> 54 us,
+// 65536 at 104 30 -> 22, the 34 calls of a 600-block Cholesky and solve 5.8 -> 4.1 ms.
+constexpr int kWide = 4;
+struct Crt4Head {
+  u64 full, done[kWide];
+  u32 tmem_slot;
+  volatile int abort;
+};
+__device__ __forceinline__ void tile_sync(int grp) { asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory"); }
+// tile_sync with the OR of pred over the tile's threads: they give up together
+__device__ __forceinline__ bool tile_sync_or(int grp, bool pred) {
+  u32 r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"((u32)pred), "r"(1 + grp)
+      : "memory");
+  return r != 0;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kThreads * kWide, 1)
+    crt4_kernel(const int16_t* __restrict__ acc, i64 ldg, i64 N, i64 j0, i64 w, i64 rows, i64 rows_per_block,
+                const int64_t* __restrict__ rowexp, const int64_t* __restrict__ colexp, int L, int n, int W, int nchunk,
+                const CrtMod* __restrict__ mods, const u32* __restrict__ negm, const uint8_t* __restrict__ ct,
+                int32_t* __restrict__ out, int64_t* __restrict__ out2, const int32_t* __restrict__ pred,
+                unsigned* __restrict__ err) {
+  if (pred && *pred == 0) return;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  Crt4Head& H = *reinterpret_cast<Crt4Head*>(base);
+  CrtMod* TB = reinterpret_cast<CrtMod*>(base + 1024);
+  u32* NM = reinterpret_cast<u32*>(base + 1024 + sizeof(CrtMod) * kNmax);
+  const int tid = threadIdx.x, warp = tid >> 5, grp = tid >> 7, lt = tid & 127;
+  uint8_t* Yh = base + kHead + (size_t)grp * 2 * kSlice;
+  uint8_t* Yl = Yh + kSlice;
+  uint8_t* table = base + kHead + (size_t)kWide * 2 * kSlice;
+  u32* col = reinterpret_cast<u32*>(Yh) + lt;
+  const i64 B = rows * w, ntiles = (B + 127) / 128;
+
+  if (tid == 0) {
+    mbar_init(&H.full, 1);
+    for (int g = 0; g < kWide; g++) mbar_init(&H.done[g], 1);
+    H.abort = 0;
+    mbar_fence_init();
+    mbar_expect_tx(&H.full, (u32)nchunk * 2 * kSlice);
+    for (u32 o = 0; o < (u32)nchunk * 2 * kSlice; o += kSlice) bulk_load(table + o, ct + o, kSlice, &H.full);
+  }
+  if (warp == 0) {
+    tmem_alloc(&H.tmem_slot, 512);
+    tmem_relinquish();
+  }
+  if (tid < 128) TB[tid] = mods[tid];
+  for (int k = tid; k < W; k += kThreads * kWide) NM[k] = negm[k];
+  __syncthreads();
+  tc_fence_after();
+  const u32 tmem = H.tmem_slot + (u32)grp * kDig;
+  const u32 taddr = tmem + ((u32)((warp & 3) * 32) << 16);
+  const u32 idesc = idesc_u8(128, kDig);
+  const int ksteps = (n + 31) / 32;
+  u32 phase = 0;
+  bool ok = mbar_wait(&H.full, 0, err);
+
+  // tiles go round the CTAs first, so that a last partial round spreads over the SMs
+  for (i64 tile = (i64)grp * gridDim.x + blockIdx.x; tile < ntiles; tile += (i64)kWide * gridDim.x) {
+    const i64 e = tile * 128 + lt;
+    const bool valid = e < B;
+    const i64 r = valid ? e / w : 0, jj = valid ? e - r * w : 0;
+    const int16_t* ap = acc + r * N + j0 + jj;
+    for (int gb = 0; gb < n; gb += 32) {
+      int v[32];
+#pragma unroll
+      for (int q = 0; q < 32; q++) v[q] = (valid && gb + q < n) ? (int)__ldcs(ap + (i64)(gb + q) * ldg) : 0;
+      store_digits(TB, gb, v, lt, Yh, Yl);
+    }
+    fence_proxy_async_smem();
+    tile_sync(grp);
+    u32 kq = 0, carry = 0, hold[32];
+    int hz = -1, ho = -1;
+    u32 hzv = 0, hov = 0, wtop = 0;
+    // word of four digit columns at word index wd (-1: the rows that give k); put(wd, word)
+    auto word = [&](const u32* z, int wd, auto put) {
+      u64 v = digit_word<false>(z);
+      if (wd < 0) {
+        kq = (u32)((v + (1u << 28)) >> 29);
+        return;
+      }
+      v += (u64)kq * NM[wd];
+      v += carry;
+      carry = (u32)(v >> 32);
+      put((u32)v);
+    };
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      if (c >= nchunk) break;
+      if (lt == 0) {
+        tc_fence_after();
+        const u32 tb = smem_u32(table) + (u32)c * 2 * kSlice, yb = smem_u32(Yh);
+        for (int h = 0; h < 2; h++)
+          for (int ks = 0; ks < ksteps; ks++) {
+            const u32 o = (u32)h * kSlice + (u32)ks * 32;
+            mma_i8(tmem, sdesc_sw128(yb + o), sdesc_sw128(tb + o), idesc, (h | ks) ? 1u : 0u);
+          }
+        mma_commit(&H.done[grp]);
+      }
+      __syncwarp();
+      ok = mbar_wait(&H.done[grp], phase, err) && ok;
+      phase ^= 1;
+      tc_fence_after();
+      const bool last = c + 1 == nchunk;
+      if (MODE == 1 && c == 1) {
+#pragma unroll
+        for (int k = 0; k < 31; k++) col[k * kThreads] = hold[k + 1];
+      }
+#pragma unroll
+      for (int c0 = 0; c0 < kDig; c0 += 32) {
+        if (c * kDig + c0 < 4 * (W + 1)) {
+          u32 z[32];
+          tmem_ld32(taddr + c0, z);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            const int wd = (c * kDig + c0) / 4 + j - 1;
+            if (wd < W)
+              word(z + 4 * j, wd, [&](u32 wv) {
+                if (MODE == 0) {
+                  if (valid) out[(i64)wd * B + e] = (int32_t)wv;
+                  if (wv != 0u) hz = wd, hzv = wv;
+                  if (wv != 0xffffffffu) ho = wd, hov = wv;
+                  wtop = wv;
+                } else if (last) {
+                  col[wd * kThreads] = wv;
+                } else {
+                  hold[c0 / 4 + j] = wv;
+                }
+              });
+          }
+        }
+      }
+      tc_fence_before();
+      if (!last) tile_sync(grp);                       // the next chunk's product overwrites the columns
+    }
+    if (valid) {
+      if (MODE == 0) {
+        const bool ng = (wtop >> 31) != 0;
+        const int k = ng ? ho : hz;
+        const u32 x = ng ? ~hov : hzv;
+        out2[e] = k < 0 ? 0 : 32 * (i64)k + 32 - __clz(x);
+      } else {
+        col_mpf_norm(col, W, rowexp[r] + colexp[(r / rows_per_block) * N + j0 + jj], L, out + e, B, out2 + e);
+      }
+    }
+    if (tile_sync_or(grp, !ok)) {                      // the columns over Y and TMEM are free again
+      H.abort = 1;
+      break;
+    }
+  }
+  if (H.abort && lt == 0) mbar_wait(&H.done[grp], phase, err);    // a wait gave up: let products drain (bounded)
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(H.tmem_slot, 512);
+}
+
+template <int MODE>
+int launch_crt4(const sdpv_ctx* c, const int16_t* acc, i64 ldg, i64 N, i64 j0, i64 w, i64 rows, i64 rpb,
+                const int64_t* rowexp, const int64_t* colexp, int L, int32_t* out, int64_t* out2, cudaStream_t st,
+                const int32_t* pred, int sms) {
+  const CtxDev& d = c->d;
+  const int nchunk = d.Epad / kDig;
+  const size_t smem = 1024 + kHead + (size_t)(kWide + nchunk) * 2 * kSlice;
+  static bool attr_set[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!attr_set[dev & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(crt4_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return set_cuda_error(e);
+    attr_set[dev & 63] = true;
+  }
+  crt4_kernel<MODE><<<(unsigned)sms, kThreads * kWide, smem, st>>>(acc, ldg, N, j0, w, rows, rpb, rowexp, colexp, L, d.n,
+                                                                  d.W, nchunk, d.crtmod, d.negm, d.ct, out, out2, pred,
+                                                                  device_error_word());
+  return launch_status();
+}
+
 template <int MODE, bool WIDE>
 int launch_crt_t(const sdpv_ctx* c, const int16_t* acc, i64 ldg, i64 N, i64 j0, i64 w, i64 rows, i64 rpb,
                  const int64_t* rowexp, const int64_t* colexp, int L, int32_t* out, int64_t* out2, cudaStream_t st,
@@ -312,6 +502,12 @@ int launch_crt(const sdpv_ctx* c, const int16_t* acc, i64 ldg, i64 N, i64 j0, i6
   const CtxDev& d = c->d;
   // at most 256 moduli (L <= 59); there 4 + E <= 512 and a word column fits the 64 ktc words of an entry in Y
   if (d.n > kNmax || d.Epad > kSlots * kDig || d.W > kWmax || d.W > 64 * d.ktc) return SDPV_EINVAL;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // more tiles than one round of two per SM: four per SM on a shared table (where it fits: n <= 128)
+  if (d.ktc == 1 && d.Epad <= 2 * kDig && d.W <= 64 && (rows * w + 127) / 128 > 2 * sms)
+    return launch_crt4<MODE>(c, acc, ldg, N, j0, w, rows, rpb, rowexp, colexp, L, out, out2, st, pred, sms);
   if (d.n > 168)
     return launch_crt_t<MODE, true>(c, acc, ldg, N, j0, w, rows, rpb, rowexp, colexp, L, out, out2, st, pred);
   return launch_crt_t<MODE, false>(c, acc, ldg, N, j0, w, rows, rpb, rowexp, colexp, L, out, out2, st, pred);

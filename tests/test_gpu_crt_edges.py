@@ -28,7 +28,7 @@ def test_float_quotient_needs_one_correction():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("L,count", [(1, 1), (8, 127), (14, 128), (26, 129), (29, 40000), (30, 40000), (39, 131),
+@pytest.mark.parametrize("L,count", [(1, 1), (8, 127), (14, 128), (26, 129), (29, 40000), (30, 40000), (39, 131), (8, 60001), (14, 76000), (26, 151552), (28, 37889),
                                      (40, 20000), (58, 700)])
 def test_crt_shapes(L, count):
     from sdpvibe_b200.mpmat import ctx
