@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kColThreads)
   const i64 i = (i64)blockIdx.x * kColThreads + threadIdx.x;
   if (i >= n) return;
   if (pred && *pred == 0) return;                      // predicated launch: O / eO untouched
-  col_mpf_add(cols + threadIdx.x, A + i, n, eA[i], Bm + i, n, eB[i], sgn, L, O + i, n, eO + i);
+  col_mpf_add(cols + threadIdx.x, PlaneSrc{A + i, n}, eA[i], PlaneSrc{Bm + i, n}, eB[i], sgn, L, O + i, n, eO + i);
 }
 
 __global__ void __launch_bounds__(kColThreads)

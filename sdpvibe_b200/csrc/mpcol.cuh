@@ -182,8 +182,23 @@ static __device__ __noinline__ int col_mul_general(const u32* a, const u32* b, i
   return s;
 }
 
-// r = a b of the entry whose operand words lie at A + k pa and B + k pb, written at O + k po (magnitude rounded
-// half up to NB = 32L - 2 bits, zero -> EZ: sdpvibe/mpf.py:58-89).  col: 2 ceil4(L) words.
+// Operand of a sum already in shared memory (a column of the same thread): copied instead of staged.
+struct ColSrc {
+  const u32* c;
+  __device__ __forceinline__ void operator()(u32* dst, int L) const {
+    for (int k = 0; k < L; k++) dst[k * T_] = c[k * T_];
+  }
+};
+// Operand in limb planes.
+struct PlaneSrc {
+  const int32_t* p;
+  i64 plane;
+  __device__ __forceinline__ void operator()(u32* dst, int L) const { col_stage(dst, p, plane, L); }
+};
+
+// r = a b of the entry whose operand words lie at A + k pa and B + k pb, written at O + k po -- limb planes, or a
+// column of the thread with po = T_ -- (magnitude rounded half up to NB = 32L - 2 bits, zero -> EZ:
+// sdpvibe/mpf.py:58-89).  col: 2 ceil4(L) words.
 //
 // Normalised operands (both magnitudes of exactly NB bits) take a short product: the result needs the product
 // from its word LM + pad - 1 up (LM = ceil4(L), the operands shifted up by pad = LM - L words), so the 4 x 4
@@ -239,11 +254,12 @@ __device__ __forceinline__ void col_mpf_mul(u32* col, const int32_t* __restrict_
 // r = a + sgn b (operands aligned at max exponent - 32 in L + 2 words, each rounded half up, then the sum
 // renormalised with its magnitude rounded half up: sdpvibe/mpf.py:92-124).  The two aligned operands are
 // formed, signed and added word by word in one pass; the sum replaces a in its column.  col: 2 L + 2 words.
-__device__ __forceinline__ void col_mpf_add(u32* col, const int32_t* A, i64 pa, i64 ea, const int32_t* B, i64 pb,
-                                            i64 eb, int sgn, int L, int32_t* O, i64 po, i64* eO) {
+template <class SrcA, class SrcB>
+__device__ __forceinline__ void col_mpf_add(u32* col, SrcA A, i64 ea, SrcB B, i64 eb, int sgn, int L, int32_t* O, i64 po,
+                                            i64* eO) {
   u32 *ca = col, *cb = col + (L + 2) * T_;
-  col_stage(ca, A, pa, L);
-  col_stage(cb, B, pb, L);
+  A(ca, L);
+  B(cb, L);
   cp_async_commit();
   cp_async_wait<0>();
   const u32 ta = ca[(L - 1) * T_], tb = cb[(L - 1) * T_];

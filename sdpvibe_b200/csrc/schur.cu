@@ -16,12 +16,12 @@
 #include <cmath>
 
 #include "common.cuh"
-#include "mpcore.cuh"
+#include "mpcol.cuh"
 
 namespace {
 using namespace sdpv;
 
-constexpr int kThreads = 128;
+constexpr int kThreads = kColThreads;
 
 __device__ __forceinline__ void seg_of(int s, int& c, int& r) {
   c = 0;
@@ -29,18 +29,14 @@ __device__ __forceinline__ void seg_of(int s, int& c, int& r) {
   r = s - c * (c + 1) / 2;
 }
 
-template <int LMAX>
-__device__ __forceinline__ void load_entry(const int32_t* __restrict__ M, const i64* __restrict__ eM, i64 plane,
-                                           i64 idx, int L, u32* w, i64& e) {
-  for (int k = 0; k < L; k++) w[k] = (u32)__ldg(M + (i64)k * plane + idx);
-  e = __ldg(eM + idx);
-}
+// words of the working columns (a product's operands, or a sum's), then three kept numbers of L words
+__host__ __device__ inline int work_words(int L) { return 2 * ((L + 3) & ~3) > 2 * L + 2 ? 2 * ((L + 3) & ~3) : 2 * L + 2; }
 
-template <int LMAX>
 __global__ void __launch_bounds__(kThreads)
     schur_kernel(int L, i64 nb, int P, int K, int dim, const int32_t* __restrict__ A, const i64* __restrict__ eA,
                  const int32_t* __restrict__ Y, const i64* __restrict__ eY, const uint8_t* __restrict__ xmask,
                  const int32_t* __restrict__ onem, i64 onee, int32_t* __restrict__ S, i64* __restrict__ eS) {
+  extern __shared__ u32 cols[];
   const i64 ntri = (i64)P * (P + 1) / 2;
   const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nb * ntri) return;
@@ -52,52 +48,55 @@ __global__ void __launch_bounds__(kThreads)
   const int j = q - i * (i + 1) / 2;
   const int W = dim * K;
   const i64 plane = 2 * nb * (i64)W * W, splane = nb * (i64)P * P;
-  u32 r[LMAX];
-  i64 er;
-  if (i == j && !xmask[b * P + i]) {
-    for (int k = 0; k < L; k++) r[k] = (u32)onem[k];
-    er = onee;
-  } else if (dim == 1) {
-    u32 x[LMAX], y[LMAX], m[2][LMAX];
-    i64 ex, ey, em[2];
-    for (int p = 0; p < 2; p++) {
-      const i64 idx = ((p * nb + b) * W + i) * W + j;
-      load_entry<LMAX>(A, eA, plane, idx, L, x, ex);
-      load_entry<LMAX>(Y, eY, plane, idx, L, y, ey);
-      mpf_mul_dev<LMAX>(x, ex, y, ey, L, m[p], em[p]);
-    }
-    mpf_add_dev<LMAX>(m[0], em[0], m[1], em[1], 1, L, r, er);
-  } else {
-    const int si = i / K, a = i - si * K, sj = j / K, bb = j - sj * K;
-    int c0, r0, c1, r1;
-    seg_of(si, c0, r0);
-    seg_of(sj, c1, r1);
-    u32 el[2][LMAX], x[LMAX], y[LMAX], tt[LMAX];
-    i64 ee[2], ex, ey, et;
-    for (int p = 0; p < 2; p++) {
-      const i64 base = (p * nb + b) * (i64)W;
-      // A[u, v] Y[w, z]: entry (u K + a, v K + bb) of AXI times entry (w K + a, z K + bb) of AY
-      auto term = [&](int u, int v, int w, int z, u32* out, i64& eo) {
-        load_entry<LMAX>(A, eA, plane, (base + u * K + a) * W + v * K + bb, L, x, ex);
-        load_entry<LMAX>(Y, eY, plane, (base + w * K + a) * W + z * K + bb, L, y, ey);
-        mpf_mul_dev<LMAX>(x, ex, y, ey, L, out, eo);
-      };
-      term(c0, r1, r0, c1, el[p], ee[p]);
-      term(r0, r1, c0, c1, tt, et);
-      mpf_add_dev<LMAX>(el[p], ee[p], tt, et, 1, L, el[p], ee[p]);
-      term(c0, c1, r0, r1, tt, et);
-      mpf_add_dev<LMAX>(el[p], ee[p], tt, et, 1, L, el[p], ee[p]);
-      term(r0, c1, c0, r1, tt, et);
-      mpf_add_dev<LMAX>(el[p], ee[p], tt, et, 1, L, el[p], ee[p]);
-    }
-    mpf_add_dev<LMAX>(el[0], ee[0], el[1], ee[1], 1, L, r, er);
-    if (er != SDPV_EZ) er -= 2;
-  }
+  u32* work = cols + threadIdx.x;
+  u32* keep = work + (size_t)work_words(L) * T_;
+  auto slot = [&](int s) { return keep + (size_t)s * L * T_; };
   const i64 o1 = (b * P + i) * (i64)P + j, o2 = (b * P + j) * (i64)P + i;
-  for (int k = 0; k < L; k++) {
-    S[(i64)k * splane + o1] = (int32_t)r[k];
-    S[(i64)k * splane + o2] = (int32_t)r[k];
+  i64 er;
+  // kept number d = entry of AXI at ia times entry of AY at iy; returns its exponent
+  auto product = [&](int d, i64 ia, i64 iy) -> i64 {
+    i64 e;
+    col_mpf_mul(work, A + ia, plane, __ldg(eA + ia), Y + iy, plane, __ldg(eY + iy), L, (int32_t*)slot(d), T_, &e);
+    return e;
+  };
+  auto sum = [&](int x, i64 ex, int y, i64 ey, int32_t* out, i64 stride) -> i64 {
+    i64 e;
+    col_mpf_add(work, ColSrc{slot(x)}, ex, ColSrc{slot(y)}, ey, 1, L, out, stride, &e);
+    return e;
+  };
+  if (i == j && !xmask[b * P + i]) {
+    for (int k = 0; k < L; k++) S[(i64)k * splane + o1] = onem[k];
+    er = onee;
+  } else {
+    i64 ee[2];
+    if (dim == 1) {
+      for (int p = 0; p < 2; p++) {
+        const i64 idx = ((p * nb + b) * W + i) * W + j;
+        ee[p] = product(p, idx, idx);
+      }
+    } else {
+      const int si = i / K, a = i - si * K, sj = j / K, bb = j - sj * K;
+      int c0, r0, c1, r1;
+      seg_of(si, c0, r0);
+      seg_of(sj, c1, r1);
+      for (int p = 0; p < 2; p++) {
+        const i64 base = (p * nb + b) * (i64)W;
+        // A[u, v] Y[w, z]: entry (u K + a, v K + bb) of AXI times entry (w K + a, z K + bb) of AY
+        auto term = [&](int d, int u, int v, int w, int z) {
+          return product(d, (base + u * K + a) * W + v * K + bb, (base + w * K + a) * W + z * K + bb);
+        };
+        ee[p] = term(p, c0, r1, r0, c1);
+        for (int x = 0; x < 3; x++) {
+          const i64 et = x == 0 ? term(2, r0, r1, c0, c1) : (x == 1 ? term(2, c0, c1, r0, r1) : term(2, r0, c1, c0, r1));
+          ee[p] = sum(p, ee[p], 2, et, (int32_t*)slot(p), T_);
+        }
+      }
+    }
+    er = sum(0, ee[0], 1, ee[1], S + o1, splane);
+    if (dim > 1 && er != SDPV_EZ) er -= 2;
   }
+  if (i != j)
+    for (int k = 0; k < L; k++) S[(i64)k * splane + o2] = S[(i64)k * splane + o1];
   eS[o1] = er;
   eS[o2] = er;
 }
@@ -111,12 +110,16 @@ extern "C" int sdpv_schur_assemble(int L, int64_t nb, int P, int K, int dim, con
   const i64 n = nb * (i64)P * (P + 1) / 2;
   if (n == 0) return SDPV_OK;
   const unsigned grid = (unsigned)((n + kThreads - 1) / kThreads);
-  cudaStream_t st = sdpv::as_stream(stream);
-  if (L <= 16)
-    schur_kernel<16><<<grid, kThreads, 0, st>>>(L, nb, P, K, dim, AXI, eAXI, AY, eAY, xmask, one_m, one_e, S, eS);
-  else if (L <= 32)
-    schur_kernel<32><<<grid, kThreads, 0, st>>>(L, nb, P, K, dim, AXI, eAXI, AY, eAY, xmask, one_m, one_e, S, eS);
-  else
-    schur_kernel<64><<<grid, kThreads, 0, st>>>(L, nb, P, K, dim, AXI, eAXI, AY, eAY, xmask, one_m, one_e, S, eS);
+  const size_t smem = (size_t)(work_words(L) + 3 * L) * kColThreads * 4, most = (size_t)(work_words(64) + 192) * kColThreads * 4;
+  static bool set[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!set[dev & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(schur_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (e != cudaSuccess) return sdpv::set_cuda_error(e);
+    set[dev & 63] = true;
+  }
+  schur_kernel<<<grid, kThreads, smem, sdpv::as_stream(stream)>>>(L, nb, P, K, dim, AXI, eAXI, AY, eAY, xmask, one_m, one_e,
+                                                                  S, eS);
   return sdpv::launch_status();
 }
