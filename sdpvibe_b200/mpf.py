@@ -411,7 +411,7 @@ def gemm(A, B, transA=False, transB=False):
     """C = op(A) op(B) (2-d, or batched 3-d (nb, ., .)); exact products, every entry rounded once
     (operands aligned per row of op(A) / column of op(B)) (sdpvibe/mpf.py:401-452)."""
     sa, sb = A.e.shape, B.e.shape
-    assert len(sa) == len(sb), (A.shape, B.shape)
+    assert len(sa) == len(sb) and len(sa) in (2, 3), (A.shape, B.shape)
     nb = sa[0] if len(sa) == 3 else 1
     M, K = (sa[-1], sa[-2]) if transA else (sa[-2], sa[-1])
     N, K2 = (sb[-2], sb[-1]) if transB else (sb[-1], sb[-2])
