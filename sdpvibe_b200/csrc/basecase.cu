@@ -1123,7 +1123,13 @@ __global__ void __launch_bounds__(kThreadsS) trinv_tiles_k(const u32* __restrict
       u32* dst = Xm + (size_t)tri(i, k) * WP;
       const u32 *xl = Lc + (size_t)i * WP, *yx = Xm + (size_t)e * WP;
       const bool add = lsj[i] == xs[e];
-      if (LF == 26 && ltj[i] <= 26 && xt[e] <= 30)
+      // tops as tight as a well scaled tile has them (|l_ij| < 1, |x_jk| < 2^32): the multiplier sets a row's time
+      // (9.8 of 13 thousand cycles at 537 multiply-adds a product), and these take 402
+      if (LF == 26 && ltj[i] <= 25 && xt[e] <= 26)
+        fx_rmw_reg2<26, 25, 26>(dst, xl, yx, add, WL);
+      else if (LF == 24 && ltj[i] <= 23 && xt[e] <= 24)
+        fx_rmw_reg2<24, 23, 24>(dst, xl, yx, add, WL);
+      else if (LF == 26 && ltj[i] <= 26 && xt[e] <= 30)
         fx_rmw_reg2<26, 26, 30>(dst, xl, yx, add, WL);
       else if (LF == 24 && ltj[i] <= 24 && xt[e] <= 28)
         fx_rmw_reg2<24, 24, 28>(dst, xl, yx, add, WL);
