@@ -115,6 +115,7 @@ int sdpv_tune_get(int knob, int* value);
  * sdpv_bigfloat_load: the records from host byte pos copied to dbuf (dbytes >= min(len - pos, n (13 + 8 nl)))
  *   while a host pass finds their offsets (offsets: n host words, relative to pos) and *end; *regular = 1 when no
  *   record is a zero record, else the offsets are copied to doffsets too.  SDPV_EINVAL if truncated/corrupt.
+ *   The stream is synchronised: buf and offsets may be reused on return.
  * sdpv_bigfloat_unpack: device records at offsets (NULL: every record 13 + 8 nl bytes) -> planar (L, n) limbs +
  *   exponents, mantissa rounded half up to at most 32 L - 2 bits (L <= 64, nl <= 64).
  * sdpv_bigfloat_pack: planar limbs + exponents -> device records at offsets (1 or 13 + 8 nl bytes each);

@@ -178,15 +178,16 @@ extern "C" int sdpv_bigfloat_load(const uint8_t* buf, int64_t len, int64_t pos, 
                        ? cudaMemcpyAsync(dbuf, buf + pos, (size_t)bytes, cudaMemcpyHostToDevice, st)
                        : cudaSuccess;
   if (worker.joinable()) worker.join();
-  if (rc != SDPV_OK) return rc;
-  if (ce != cudaSuccess) return sdpv::set_cuda_error(ce);
-  *regular = *end == most;
-  *end += pos;
-  if (!*regular) {
-    ce = cudaMemcpyAsync(doffsets, offsets, (size_t)n * 8, cudaMemcpyHostToDevice, st);
-    if (ce != cudaSuccess) return sdpv::set_cuda_error(ce);
+  if (rc == SDPV_OK && ce == cudaSuccess) {
+    *regular = *end == most;
+    *end += pos;
+    if (!*regular) ce = cudaMemcpyAsync(doffsets, offsets, (size_t)n * 8, cudaMemcpyHostToDevice, st);
   }
-  return SDPV_OK;
+  // both copies may read pinned memory asynchronously; the caller may reuse buf and offsets on return
+  const cudaError_t cs = cudaStreamSynchronize(st);
+  if (rc != SDPV_OK) return rc;
+  if (ce == cudaSuccess) ce = cs;
+  return ce == cudaSuccess ? SDPV_OK : sdpv::set_cuda_error(ce);
 }
 
 extern "C" int sdpv_bigfloat_unpack(const uint8_t* buf, const int64_t* offsets, int64_t n, int nl, int L, int32_t* out,

@@ -38,18 +38,20 @@ def decode_bigfloats(buf, pos, n, nl, L):
     if n == 0:
         return MPF(torch.zeros((L, 0), dtype=torch.int32, device=dev),
                    torch.zeros((0,), dtype=torch.int64, device=dev)), pos
+    if n > max(0, len(arr) - pos):                                  # a record has at least its flag byte
+        raise ValueError("truncated or corrupt binary block data")
     offs = np.empty(n, dtype=np.int64)
     end, regular = ctypes.c_int64(0), ctypes.c_int(0)
     size = max(0, min(len(arr) - pos, n * (13 + 8 * nl)))
     dbuf = torch.empty((size,), dtype=torch.uint8, device=dev)
     doffs = torch.empty((n,), dtype=torch.int64, device=dev)
-    m = torch.empty((L, n), dtype=torch.int32, device=dev)
-    e = torch.empty((n,), dtype=torch.int64, device=dev)
     st = _lib.lib().sdpv_bigfloat_load(arr.ctypes.data, len(arr), pos, n, nl, dbuf.data_ptr(), size, offs.ctypes.data,
                                        doffs.data_ptr(), ctypes.byref(regular), ctypes.byref(end), _lib.stream())
     if st == _lib.EINVAL:
         raise ValueError("truncated or corrupt binary block data")
     _lib.check(st, "sdpv_bigfloat_load")
+    m = torch.empty((L, n), dtype=torch.int32, device=dev)
+    e = torch.empty((n,), dtype=torch.int64, device=dev)
     _lib.call("sdpv_bigfloat_unpack", dbuf.data_ptr(), None if regular.value else doffs.data_ptr(), n, nl, L, _lib.ptr(m),
               _lib.ptr(e), _lib.stream())
     return MPF(m, e), int(end.value)

@@ -36,3 +36,26 @@ def test_round_trip(n, zeros):
         bad[last + 1:last + 5] = (nl + 1).to_bytes(4, "little")      # |size| > nl in the last record
         with pytest.raises(ValueError):
             decode_bigfloats(bytes(bad), 11, n, nl, L)
+
+
+def test_pinned_buffer_is_free_on_return():
+    """A pinned buffer overwritten right after the call: the records read are those of the call."""
+    from sdpvibe_b200 import mpf
+    from sdpvibe_b200.sdp_io import decode_bigfloats, encode_bigfloats
+    L, nl, n = 26, 18, 400000
+    rec = encode_bigfloats(mpf.from_float(torch.arange(1.0, n + 1.0, dtype=torch.float64, device="cuda"), L), nl)
+    buf = torch.empty((len(rec),), dtype=torch.uint8, pin_memory=True)
+    arr = buf.numpy()
+    arr[:] = np.frombuffer(rec, dtype=np.uint8)
+    A, _ = decode_bigfloats(rec, 0, n, nl, L)
+    for _ in range(3):
+        B, _ = decode_bigfloats(arr, 0, n, nl, L)
+        arr[-(1 << 20):] = 0
+        assert torch.equal(A.m, B.m) and torch.equal(A.e, B.e)
+        arr[:] = np.frombuffer(rec, dtype=np.uint8)
+
+
+def test_count_beyond_the_buffer():
+    from sdpvibe_b200.sdp_io import decode_bigfloats
+    with pytest.raises(ValueError):
+        decode_bigfloats(b"\x01" * 64, 0, 1 << 36, 18, 26)
