@@ -379,10 +379,12 @@ def _align_rows(A):
     return out.view(A.m.shape), E.view(A.shape[:-1])
 
 
-# Entries of A from which one or two columns are multiplied without residues (_gemm_tall; three or four, two passes
-# over A: from four times as many).  Measured at L = 26, without / through residues: 200 x 1000 by one column 59 /
-# 85 us, 2000 x 128 99 / 102, 256 x 256 58 / 53; by three 1000 x 1000 230 / 244, 600 x 600 165 / 130.
-TALL_MIN = 1 << 17
+# Entries of A from which one or two columns are multiplied without residues (_gemm_tall), its sides at least 128.
+# Time without over time through residues at L = 5-32, K x M (K summed over): one column 2048 x 128 0.6-0.94, 512 x
+# 512 0.44-0.67, 2048 x 2048 0.19-0.32; two 128 x 2048 0.68-0.96, 2048 x 128 0.71-1.00, 2048 x 2048 0.32-0.41, but
+# 512 x 256 up to 1.06, 32 x 32768 1.05-1.09 and 8 x 16384 1.1-1.2 (the partial digit sums outweigh A).  Three or
+# four are two passes over A: 2048 x 1000 0.53-0.82, 512 x 8192 0.52-0.90, 512 x 2048 up to 1.09, 128 x 32768 1.26.
+TALL_MIN = 1 << 18
 
 
 def _gemm_tall(A, B, L, M, K, N, transB):
@@ -421,7 +423,8 @@ def gemm(A, B, transA=False, transB=False):
     shape = (nb, M, N) if len(sa) == 3 else (M, N)
     if not (nb and M and N and K):
         return zeros(shape, L)                                      # no entries, or empty sums
-    if transA and nb == 1 and N <= 4 and M * K >= TALL_MIN * (1 if N <= 2 else 4):
+    kmin, least = (128, TALL_MIN) if N <= 2 else (512, 8 * TALL_MIN)
+    if transA and nb == 1 and N <= 4 and M >= 128 and K >= kmin and M * K >= least:
         C = _gemm_tall(A, B, L, M, K, N, transB)
         if C is not None:
             return C.reshape(*shape)
