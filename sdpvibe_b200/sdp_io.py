@@ -28,6 +28,12 @@ _SIG = b"serialization::archive"
 _BIGFLOAT_CLASS = b"\0\x01\0\0\0"               # El::BigFloat class information, version 1
 
 
+# a bytes object of uninitialised contents: the records are copied from the device straight into it
+# (66000 records of 157 bytes: 7.7 -> 0.93 ms; a host tensor and a copy of it were two fresh buffers a call)
+_new_bytes = ctypes.PYFUNCTYPE(ctypes.py_object, ctypes.c_void_p, ctypes.c_ssize_t)(
+    ("PyBytes_FromStringAndSize", ctypes.pythonapi))
+
+
 def limbs_for_precision(precision):
     """GMP limbs of an mpf_t of `precision` bits as the archive stores them (__GMPF_BITS_TO_PREC + 1)"""
     return (precision + 127) // 64 + 1
@@ -74,7 +80,10 @@ def encode_bigfloats(A, nl):
     _lib.call("sdpv_bigfloat_pack", _lib.ptr(m), _lib.ptr(e), n, L, nl, _lib.ptr(offs), _lib.ptr(out), _lib.stream())
     if _lib.device_error_flags() & _lib.ERR_OVERFLOW:
         raise ValueError("cannot encode (mantissa larger than the archive precision)")
-    return out.cpu().numpy().tobytes()
+    rec = _new_bytes(None, total)                                   # filled by the device copy before anyone sees it
+    torch.frombuffer((ctypes.c_uint8 * total).from_address(np.frombuffer(rec, np.uint8).ctypes.data),
+                     dtype=torch.uint8).copy_(out)
+    return rec
 
 
 class BinReader:
