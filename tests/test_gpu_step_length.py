@@ -122,6 +122,32 @@ def test_eig_sym_f64_kernel(n):
     assert np.all(np.diff(wd, axis=1) >= 0)
 
 
+@pytest.mark.parametrize("n", [2, 6, 8, 15, 16, 22, 44, 46, 90])
+def test_eig_sym_f64_many_blocks(n):
+    """sdpv_eig_sym_f64 where the 2 x 2 sub-blocks just fill the CTA's warps, leave lanes idle, or take further rounds of
+    its threads; 400 blocks at once: LAPACK's eigenvalues within the bounds, and each block as when it is alone"""
+    from sdpvibe_b200 import _lib
+    rng = np.random.default_rng(n)
+    nb = 400
+    A = rng.standard_normal((nb, n, n))
+    A = A + np.swapaxes(A, 1, 2)
+
+    def run(B):
+        k = B.shape[0]
+        Bd = torch.from_numpy(np.ascontiguousarray(B)).cuda()
+        w = torch.empty((k, n), dtype=torch.float64, device="cuda")
+        err = torch.empty((k,), dtype=torch.float64, device="cuda")
+        _lib.call("sdpv_eig_sym_f64", _lib.ptr(Bd), k, n, _lib.ptr(w), _lib.ptr(err), None, _lib.stream())
+        return w.cpu().numpy(), err.cpu().numpy()
+
+    w, err = run(A)
+    lap = (n + 2) * 2.0 ** -52 * np.sqrt((A * A).sum(axis=(1, 2)))
+    assert np.all(np.abs(w - np.linalg.eigvalsh(A)) <= (err + lap)[:, None])
+    for q in (0, 147, 399):
+        wq, eq = run(A[q:q + 1])
+        assert np.array_equal(wq[0], w[q]) and eq[0] == err[q]
+
+
 def test_min_eig_matrix_matches_oracle():
     """M = L^-1 dM L^-T, the matrix whose float64 copy feeds the eigensolver, is bit-identical to the
     oracle's (so the float64 eigenvalues, and the step, are the reference's)."""
