@@ -285,6 +285,10 @@ __device__ void wmul_core(const u32* x, int tx, const u32* y, int ty, int t, int
 // reductions and votes, whose uniform results keep reconvergence out of the loops and branches they bound.
 // Words go in groups of four, the next group's loads issued ahead of this group's multiply-adds.  Groups of
 // eight (398 us) and one call site for the Newton chain's three products (410-456 us) were slower.
+// Above 64 words (NPL = 3) a product has up to 75 columns; each further 32 start at the first word of x that y's top word
+// still reaches: with all words of x in each, the factor of one tile took 1.84 ms at L = 70 and 1.42 at L = 60 (now 1.78
+// and 1.40; wmul_core 1.79, 1.41).  At up to 64 words the few further columns gain 1-4 % of the factor at L = 28-40, and
+// keeping the range in registers costs 1 % at L <= 26: not taken.
 //   x: 16-byte aligned, zero from tx + 1 to the end of tx's group of four and below la within la's group
 //   y: word 0 of a padded buffer (kPadLo / kPadHi), zero below lb and above ty
 template <int NPL>
@@ -299,7 +303,8 @@ __device__ __forceinline__ void wmul_pad(const u32* x, int tx, int la, const u32
                                          u32 (&m)[NPL]) {
   const int lane = threadIdx.x & 31;
   const int kmin = max(LF - 2, la + lb), kmax = tx + ty;
-  const int ncol = kmax + 2 - kmin + 1, ibase = la & ~3, ng = (tx >> 2) - (la >> 2) + 1;
+  const int ncol = kmax + 2 - kmin + 1;
+  int ibase = la & ~3, ng = (tx >> 2) - (la >> 2) + 1;
 #pragma unroll
   for (int c = 0; c < NPL; c++) m[c] = 0u;
   u32 p_c1 = 0, p_c2a = 0, p_c2b = 0, p_h = 0, cin = 0;          // carried over from the previous 32 columns
@@ -350,6 +355,10 @@ __device__ __forceinline__ void wmul_pad(const u32* x, int tx, int la, const u32
       p_c2b = __shfl_sync(kFull, c2, 31);
       p_h = __shfl_sync(kFull, h, 31);
       cin = cout;
+      if (NPL > 2) {
+        ibase = max(la, kmin + q0 + 32 - ty) & ~3;               // below, the next 32 columns meet zeros of y only
+        ng = (tx >> 2) - (ibase >> 2) + 1;
+      }
     }
   }
 }
