@@ -122,13 +122,14 @@ __device__ __forceinline__ void align_digits(u32* col, int stride, int L, i64 s6
 // of the aligned entry (zero outside its 4 L digits).  32 entries per CTA.
 constexpr int kPrep = 32, kZPad = 160;       // zero bytes around an entry's digits: indices -159 .. 16 nh - 1
 __global__ void __launch_bounds__(128) mv_prep_kernel(const int32_t* __restrict__ B, const i64* __restrict__ eB, int L,
-                                                      i64 K, i64 N, i64 ks, i64 ns, const i64* __restrict__ Eb,
-                                                      uint8_t* __restrict__ F, unsigned* err) {
-  // entry (k, n) at k ks + n ns; plane stride K N
+                                                      i64 K, i64 N, i64 ks, i64 ns, i64 n0,
+                                                      const i64* __restrict__ Eb, uint8_t* __restrict__ F,
+                                                      unsigned* err) {
+  // entry (k, n) at k ks + n ns; plane stride K N; columns n0 + blockIdx.y
   extern __shared__ __align__(16) u32 sm[];
   const MvShape sh = mv_shape(L);
   const int tid = threadIdx.x;
-  const i64 n = blockIdx.y, k0 = (i64)blockIdx.x * kPrep;
+  const i64 n = n0 + blockIdx.y, k0 = (i64)blockIdx.x * kPrep;
   const int zw = (2 * kZPad + 16 * sh.nh + 15) / 16 * 4 + 1;         // words per entry (odd pitch)
   u32* raw = sm;                                                     // [L + 1][32]
   u32* z = sm + (L + 1) * kPrep;                                           // [32][zw], digit d at byte kZPad + d
@@ -153,7 +154,7 @@ __global__ void __launch_bounds__(128) mv_prep_kernel(const int32_t* __restrict_
   __syncthreads();
   const int per = 2 * sh.nc * 8;                                     // 16-byte rows of an image
   const i64 left = K - k0 < kPrep ? K - k0 : kPrep;
-  uint4* out = reinterpret_cast<uint4*>(F + (n * K + k0) * mv_image(L));
+  uint4* out = reinterpret_cast<uint4*>(F + (blockIdx.y * K + k0) * mv_image(L));
   for (int i = tid; i < (int)left * per; i += 128) {
     const int e = i / per, j = i - e * per, r = j & 7, m = (j >> 3) % sh.nc, p = (j >> 3) / sh.nc;
     const int o = kZPad + 16 * sh.nh - 1 - 8 * p - r - 16 * m - 15;  // the 16 bytes o .. o + 15, reversed
@@ -427,6 +428,10 @@ void mv_split(int L, i64 K, i64 M, i64& kper, int& nrange) {
   nrange = (int)((K + kper - 1) / kper);
 }
 
+// Columns whose Toeplitz images the workspace holds: all N where they take at most a quarter of A's bytes, else the two that
+// are worked at once (5.4 KB per value of k and column at L = 26: four columns of 65536 x 128 would take more than A).
+i64 image_columns(int L, i64 M, i64 N) { return N <= 2 || 4 * N * mv_image(L) <= M * (4 * L + 8) ? N : 2; }
+
 }  // namespace
 
 // Bytes of workspace of sdpv_gemm_tall (0: the shape is not taken).
@@ -436,8 +441,9 @@ extern "C" int sdpv_gemm_tall_workspace(int L, int64_t M, int64_t K, int64_t N, 
   if (L < 1 || L > kLmax || M < 1 || K < 1 || K > 65536 || N < 1 || N > 4) return SDPV_OK;
   i64 kper;
   int nrange;
+  const int nc = N > 1 ? 2 : 1;                                        // columns worked at once
   mv_split(L, K, M, kper, nrange);
-  *bytes = round_up(N * K * mv_image(L), 256) + (N > 1 ? 2 : 1) * (i64)nrange * 16 * mv_shape(L).nh * round_up(M, kRows) * 4;
+  *bytes = round_up(image_columns(L, M, N) * K * mv_image(L), 256) + nc * (i64)nrange * 16 * mv_shape(L).nh * round_up(M, kRows) * 4;
   return SDPV_OK;
 }
 
@@ -451,7 +457,8 @@ extern "C" int sdpv_gemm_tall(const int32_t* Am, const int64_t* Ae, const int32_
   unsigned* err = sdpv::device_error_word();
   const MvShape sh = mv_shape(L);
   uint8_t* F = static_cast<uint8_t*>(ws);
-  int32_t* part = reinterpret_cast<int32_t*>(F + round_up(N * K * mv_image(L), 256));
+  const i64 images = image_columns(L, M, N);
+  int32_t* part = reinterpret_cast<int32_t*>(F + round_up(images * K * mv_image(L), 256));
   i64 kper;
   int nrange;
   mv_split(L, K, M, kper, nrange);
@@ -497,12 +504,13 @@ extern "C" int sdpv_gemm_tall(const int32_t* Am, const int64_t* Ae, const int32_
     if (e != cudaSuccess) return sdpv::set_cuda_error(e);
     set[dev & 63] = true;
   }
-  mv_prep_kernel<<<dim3((unsigned)((K + kPrep - 1) / kPrep), (unsigned)N), 128, sm_prep, st>>>(
-      Bm, Be, L, K, N, transB ? 1 : N, transB ? K : 1, Eb, F, err);
   const dim3 grid((unsigned)(Mp / kRows), (unsigned)nrange);
   for (i64 n = 0; n < N;) {
     const int nc = n + 1 < N ? 2 : 1;                                  // two columns at once
-    const uint8_t* Fn = F + n * K * mv_image(L);
+    if (n % images == 0)
+      mv_prep_kernel<<<dim3((unsigned)((K + kPrep - 1) / kPrep), (unsigned)(images < N - n ? images : N - n)), 128, sm_prep,
+                       st>>>(Bm, Be, L, K, N, transB ? 1 : N, transB ? K : 1, n, Eb, F, err);
+    const uint8_t* Fn = F + n % images * K * mv_image(L);
     if (nc == 2)
       mv_main_kernel<2><<<grid, kThreads, sm_main(2), st>>>(mm, me, tma, Am, Ae, L, K, M, Ea, Fn, kper, Mp, slots(2), part,
                                                         part_col, err);

@@ -37,6 +37,21 @@ def test_toeplitz_layout(L):
         assert total == v * x
 
 
+def _workspace(L, M, K, N):
+    import ctypes
+    from sdpvibe_b200 import _lib
+    need = ctypes.c_int64()
+    assert _lib.lib().sdpv_gemm_tall_workspace(L, M, K, N, ctypes.byref(need)) == 0
+    return need.value
+
+
+@pytest.mark.parametrize("L,M,K,N", [(32, 128, 65536, 4), (26, 128, 65536, 3), (26, 1000, 7380, 4), (26, 600, 7380, 4), (8, 128, 4096, 4)])
+def test_workspace_stays_below_the_matrix(L, M, K, N):
+    """the columns' images are held in pairs where all of them would take more than a quarter of the matrix"""
+    assert _workspace(L, M, K, N) < K * M * (4 * L + 8)
+    assert _workspace(L, M, K, N) <= max(_workspace(L, M, K, 2), K * M * (4 * L + 8) / 4 + _workspace(L, M, K, 2))
+
+
 def _rand(shape, L, seed):
     import torch
     from sdpvibe_b200 import mpf
