@@ -417,15 +417,29 @@ __global__ void __launch_bounds__(1024) mv_finish_kernel(const int32_t* __restri
 
 i64 round_up(i64 a, i64 b) { return (a + b - 1) / b * b; }
 
-// Ranges of k per block of columns: enough CTAs for one per SM, no more values of k than int32 sums hold.
-void mv_split(int L, i64 K, i64 M, i64& kper, int& nrange) {
-  const i64 blocks = (M + kRows - 1) / kRows, most = 32000 / L;
-  i64 want = 148 / blocks;
-  if (want < 1) want = 1;
-  kper = (K + want - 1) / want;
-  if (kper < 16) kper = 16;
-  if (kper > most) kper = most;
-  nrange = (int)((K + kper - 1) / kper);
+// Ranges of k per block of columns, for nc columns at once.  A CTA fills an SM, so blocks * nrange CTAs run in rounds of
+// one per SM; the time of a round's steps against that of a range's digit sums, written and read back, decides (us,
+// fitted to 1 .. 296 ranges of twelve sizes at L = 6, 16, 26, 32).  One range per block left SMs idle from 75 blocks of
+// columns on: 10000 x 1000 at L = 26 835 -> 604 us (5 ranges), four columns 2145 -> 1620.  No more values of k than int32
+// sums hold.
+void mv_split(int L, i64 K, i64 M, int nc, i64& kper, int& nrange) {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const i64 blocks = (M + kRows - 1) / kRows, least = (K + 32000 / L - 1) / (32000 / L), most = (K + 15) / 16;
+  const double step = 0.38 + 0.0155 * L + (nc - 1) * 0.012 * L, start = 3.0;
+  const double sums = nc * (double)(blocks * kRows) * (9e-5 * mv_shape(L).nh + 2.3e-4);
+  double best = 1e300;
+  kper = K;
+  nrange = 1;
+  for (int rounds = 0; rounds <= 8; rounds++) {                      // the most ranges in so many rounds
+    i64 r = rounds * (i64)sms / blocks;
+    r = r > most ? most : r;
+    r = r < least ? least : r;
+    const i64 k = (K + r - 1) / r, n = (K + k - 1) / k;
+    const double cost = (double)((blocks * n + sms - 1) / sms) * ((double)k * step + start) + sums * (double)n;
+    if (cost < best) best = cost, kper = k, nrange = (int)n;
+  }
 }
 
 // Columns whose Toeplitz images the workspace holds: all N where they take at most a quarter of A's bytes, else the two that
@@ -442,7 +456,7 @@ extern "C" int sdpv_gemm_tall_workspace(int L, int64_t M, int64_t K, int64_t N, 
   i64 kper;
   int nrange;
   const int nc = N > 1 ? 2 : 1;                                        // columns worked at once
-  mv_split(L, K, M, kper, nrange);
+  mv_split(L, K, M, nc, kper, nrange);
   *bytes = round_up(image_columns(L, M, N) * K * mv_image(L), 256) + nc * (i64)nrange * 16 * mv_shape(L).nh * round_up(M, kRows) * 4;
   return SDPV_OK;
 }
@@ -461,7 +475,7 @@ extern "C" int sdpv_gemm_tall(const int32_t* Am, const int64_t* Ae, const int32_
   int32_t* part = reinterpret_cast<int32_t*>(F + round_up(images * K * mv_image(L), 256));
   i64 kper;
   int nrange;
-  mv_split(L, K, M, kper, nrange);
+  mv_split(L, K, M, N > 1 ? 2 : 1, kper, nrange);
   const i64 Mp = round_up(M, kRows);
   const int zw = (2 * kZPad + 16 * sh.nh + 15) / 16 * 4 + 1;
   const size_t sm_prep = (size_t)(L + 1 + zw) * kPrep * 4;

@@ -380,10 +380,12 @@ def _align_rows(A):
 
 
 # Entries of A from which one or two columns are multiplied without residues (_gemm_tall), its sides at least 128.
-# Time without over time through residues at L = 5-32, K x M (K summed over): one column 2048 x 128 0.6-0.94, 512 x
-# 512 0.44-0.67, 2048 x 2048 0.19-0.32; two 128 x 2048 0.68-0.96, 2048 x 128 0.71-1.00, 2048 x 2048 0.32-0.41, but
-# 512 x 256 up to 1.06, 32 x 32768 1.05-1.09 and 8 x 16384 1.1-1.2 (the partial digit sums outweigh A).  Three or
-# four are two passes over A: 2048 x 1000 0.53-0.82, 512 x 8192 0.52-0.90, 512 x 2048 up to 1.09, 128 x 32768 1.26.
+# Time without over time through residues at L = 5-32, M x K (K summed over): one column 2048 x 128 0.45-0.67, 512 x
+# 512 0.44-0.68, 128 x 2048 0.59-0.93; two 128 x 2048 0.71-1.01, 2048 x 128 0.67-0.96, 1024 x 256 0.58-0.81; below, 256 x
+# 512 up to 1.06, 32768 x 32 1.05-1.09 and 16384 x 8 1.1-1.2 (the partial digit sums outweigh A).  Three or four are two
+# passes over A, from 8 times as many entries and K = 512 on: 4096-19000 x 512 three 0.57-0.91, four 0.65-0.90; where the
+# residue path is at its best (L = 17-29: up to 128 moduli, one full operand tile an entry) four 0.90-1.06 at K = 512,
+# 0.93-0.98 at 576, 0.83-0.98 at 600.  Below, 2048 x 512 up to 1.09, 32768 x 128 1.26.
 TALL_MIN = 1 << 18
 
 
@@ -423,7 +425,7 @@ def gemm(A, B, transA=False, transB=False):
     shape = (nb, M, N) if len(sa) == 3 else (M, N)
     if not (nb and M and N and K):
         return zeros(shape, L)                                      # no entries, or empty sums
-    kmin, least = (128, TALL_MIN) if N <= 2 else (512, 8 * TALL_MIN)
+    kmin, least = (128, TALL_MIN) if N <= 2 else (576 if N == 4 and 16 < L < 30 else 512, 8 * TALL_MIN)
     if transA and nb == 1 and N <= 4 and M >= 128 and K >= kmin and M * K >= least:
         C = _gemm_tall(A, B, L, M, K, N, transB)
         if C is not None:

@@ -52,6 +52,22 @@ def test_workspace_stays_below_the_matrix(L, M, K, N):
     assert _workspace(L, M, K, N) <= max(_workspace(L, M, K, 2), K * M * (4 * L + 8) / 4 + _workspace(L, M, K, 2))
 
 
+@pytest.mark.parametrize("L", [5, 26, 32])
+@pytest.mark.parametrize("M", [1000, 6400, 9600, 10000, 12000, 15000, 18800, 19000, 40000])
+@pytest.mark.parametrize("K", [1000, 7380])
+def test_split_fills_the_processors(L, M, K):
+    """blocks of 128 columns times ranges of k: the rounds of one CTA per SM (148) take at most 1.35 times the steps
+    that an even split would (one range per block: up to 1.97), and no range has more values of k than int32 sums hold"""
+    nh = 2 * ((L + 3) // 4)
+    image = 2 * (2 * ((4 * L + 31) // 32) + nh - 1) * 128
+    blocks = (M + 127) // 128
+    ranges, rest = divmod(_workspace(L, M, K, 1) - (K * image + 255) // 256 * 256, 16 * nh * blocks * 128 * 4)
+    assert rest == 0
+    kper = -(-K // ranges)
+    assert kper <= 32000 // L
+    assert -(-blocks * ranges // 148) * kper <= 1.35 * blocks * K / 148
+
+
 def _rand(shape, L, seed):
     import torch
     from sdpvibe_b200 import mpf
@@ -73,7 +89,8 @@ def _rand(shape, L, seed):
 @pytest.mark.parametrize("L,M,K,N,tB", [(1, 5, 3, 1, False), (2, 130, 40, 2, True), (8, 33, 2100, 4, False),
                                         (26, 1000, 530, 1, False), (26, 257, 300, 3, True), (26, 1, 5000, 1, False),
                                         (31, 128, 64, 2, False), (32, 129, 1100, 1, True), (10, 64, 65536, 1, False),
-                                        (24, 20000, 17, 1, False), (26, 130, 900, 2, False), (29, 132, 700, 3, True)])
+                                        (24, 20000, 17, 1, False), (26, 130, 900, 2, False), (29, 132, 700, 3, True),
+                                        (26, 10000, 200, 4, False), (5, 12001, 130, 3, True)])
 def test_tall_matches_residue_path(monkeypatch, L, M, K, N, tB):
     import torch
     from sdpvibe_b200 import mpf
