@@ -23,6 +23,7 @@
 // 48 -> 30 us, 1000 entries 37 -> 15 us; crt_block of 1024 entries 22 -> 15 us.  Two CTAs per SM, one tile each
 // (102 KB at 116 moduli): the table twice on the SM costs less than two tiles waiting for one another.
 #include "common.cuh"
+#include "crt_reduce.h"
 #include "mpcol.cuh"
 
 namespace {
@@ -63,12 +64,10 @@ __device__ __forceinline__ void store_digits(const CrtMod* TB, int gb, const int
       for (int u = 0; u < 4; u++) {
         const int a = v[16 * h + 4 * q4 + u];
         const int4 c = *reinterpret_cast<const int4*>(&TB[gb + 16 * h + 4 * q4 + u]);
-        // x = a inv, q = round(x / m) from the float product (off by less than 0.002): |x - q m| <= 0.502 m, so one
-        // correction gives y in [0, m)
+        // q = round(a inv / m) from the float product (off by less than 0.002)
         const float fa = __int_as_float(0x4B008000 + a) - 8421376.0f;
         const int qb = __float_as_int(fmaf(fa, __int_as_float(c.z), 12582912.0f));
-        const int x = a * c.y + c.w - qb * c.x;
-        y[u] = (u32)(x + ((x >> 31) & c.x));
+        y[u] = crt_reduce((u32)a, (u32)c.y, (u32)c.x, (u32)c.w, (u32)qb);
       }
       const u32 p01 = y[0] + (y[1] << 16), p23 = y[2] + (y[3] << 16);
       ph[q4] = __byte_perm(p01 >> 7, p23 >> 7, 0x6420);
