@@ -143,6 +143,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   const u32 idesc = idesc_u8(128, kDig);
   const int ksteps = (n + 31) / 32;
   u32 seq = 0, phase = 0;                              // chunks used so far, parity of `done`
+  u32 loads = nslot;                                   // thread 32: table copies issued
 
   while (true) {
     // ---- pre-pass: the digits of y_i
@@ -189,6 +190,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         const bool last = tile + gridDim.x >= ntiles;
         const u32 nx = (u32)c + nslot;        // < 2 nchunk
         if (nx >= (u32)nchunk && last) continue;
+        loads = seq + nslot + 1;
         mbar_expect_tx(&H.full[s], cbytes);
         const uint8_t* src = ct + (size_t)(nx % nchunk) * cbytes;
         for (u32 o = 0; o < cbytes; o += kSlice) bulk_load(slots + s * cbytes + o, src + o, kSlice, &H.full[s]);
@@ -260,7 +262,12 @@ __global__ void __launch_bounds__(kThreads, 2)
     if (H.abort) break;
   }
   __syncthreads();
-  if (H.abort && tid == 0) mbar_wait(&H.done, phase, err);   // a wait gave up: let committed products drain (bounded)
+  if (H.abort && tid == 0) mbar_wait(&H.done, phase ^ 1u, err);   // a wait gave up: let products and copies drain (bounded)
+  if (H.abort && tid == 32)
+    for (int s = 0; s < nslot; s++) {
+      const int p = last_load_parity(loads, nslot, s);
+      if (p >= 0) mbar_wait(&H.full[s], (u32)p, err);
+    }
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, tcols);
 }
@@ -274,7 +281,6 @@ constexpr int kWide = 4;
 struct Crt4Head {
   u64 full, done[kWide];
   u32 tmem_slot;
-  volatile int abort;
 };
 __device__ __forceinline__ void tile_sync(int grp) { asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory"); }
 // tile_sync with the OR of pred over the tile's threads: they give up together
@@ -286,6 +292,15 @@ __device__ __forceinline__ bool tile_sync_or(int grp, bool pred) {
       : "r"((u32)pred), "r"(1 + grp)
       : "memory");
   return r != 0;
+}
+
+// Waits once more where the bounded wait gives up (the error bit is set): copies and products get that time to land before
+// the CTA goes on or ends.  Inlined in MODE 0 and a call in MODE 1: the kernel uses all 128 registers, and the other way
+// round the loop's schedule suffers (400000 entries at 116 moduli: 143 instead of 123 us, 112 instead of 110).
+__device__ __noinline__ bool mbar_again(u64* bar, u32 phase, unsigned* err) { return mbar_wait(bar, phase, err); }
+template <int MODE>
+__device__ __forceinline__ bool mbar_drain(u64* bar, u32 phase, unsigned* err) {
+  return mbar_wait(bar, phase, err) || (MODE == 0 ? mbar_wait(bar, phase, err) : mbar_again(bar, phase, err));
 }
 
 template <int MODE>
@@ -311,7 +326,6 @@ __global__ void __launch_bounds__(kThreads * kWide, 1)
   if (tid == 0) {
     mbar_init(&H.full, 1);
     for (int g = 0; g < kWide; g++) mbar_init(&H.done[g], 1);
-    H.abort = 0;
     mbar_fence_init();
     mbar_expect_tx(&H.full, (u32)nchunk * 2 * kSlice);
     for (u32 o = 0; o < (u32)nchunk * 2 * kSlice; o += kSlice) bulk_load(table + o, ct + o, kSlice, &H.full);
@@ -329,7 +343,7 @@ __global__ void __launch_bounds__(kThreads * kWide, 1)
   const u32 idesc = idesc_u8(128, kDig);
   const int ksteps = (n + 31) / 32;
   u32 phase = 0;
-  bool ok = mbar_wait(&H.full, 0, err);
+  bool ok = mbar_drain<MODE>(&H.full, 0, err);
 
   // tiles go round the CTAs first, so that a last partial round spreads over the SMs
   for (i64 tile = (i64)grp * gridDim.x + blockIdx.x; tile < ntiles; tile += (i64)kWide * gridDim.x) {
@@ -374,7 +388,7 @@ __global__ void __launch_bounds__(kThreads * kWide, 1)
         mma_commit(&H.done[grp]);
       }
       __syncwarp();
-      ok = mbar_wait(&H.done[grp], phase, err) && ok;
+      ok = mbar_drain<MODE>(&H.done[grp], phase, err) && ok;
       phase ^= 1;
       tc_fence_after();
       const bool last = c + 1 == nchunk;
@@ -420,12 +434,8 @@ __global__ void __launch_bounds__(kThreads * kWide, 1)
         col_mpf_norm(col, W, rowexp[r] + colexp[(r / rows_per_block) * N + j0 + jj], L, out + e, B, out2 + e);
       }
     }
-    if (tile_sync_or(grp, !ok)) {                      // the columns over Y and TMEM are free again
-      H.abort = 1;
-      break;
-    }
+    if (tile_sync_or(grp, !ok)) break;                 // (else) the columns over Y and TMEM are free again
   }
-  if (H.abort && lt == 0) mbar_wait(&H.done[grp], phase, err);    // a wait gave up: let products drain (bounded)
   __syncthreads();
   if (warp == 0) tmem_dealloc(H.tmem_slot, 512);
 }
