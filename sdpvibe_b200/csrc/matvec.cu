@@ -239,6 +239,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_after();
   const u32 tmem = S.tmem_slot;
   const int nn = 8 * sh.nh;                                          // columns per parity
+  int loaded = 0;                                                    // the loading thread: images issued
 
   if (warp < 4 * kGroups) {
     // aligners: group g takes steps g, g + kGroups, ...; thread = row (column i of A)
@@ -307,8 +308,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else if (tid == 128 * kGroups + 32) {
     // Toeplitz operands: image n into slot n mod nf once the products of step n - nf have read it
     const uint8_t* src = F + k0 * (i64)fbytes;
-    int fs = 0, round = 0, n = 0;
-    for (; n < steps && !S.abort; n++) {
+    int fs = 0, round = 0;
+    for (int n = 0; n < steps && !S.abort; n++) {
       if (round > 0 && !mbar_wait(&S.fempty[fs], (round - 1) & 1, err)) {
         S.abort = 1;
         break;
@@ -317,9 +318,9 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
       for (int c = 0; c < NC; c++)                                   // column c's images follow K images later
         bulk_load(fsm + (fs * NC + c) * fbytes, src + ((i64)c * K + n) * fbytes, fbytes, &S.ffull[fs]);
+      loaded = n + 1;
       if (++fs == nf) fs = 0, round++;
     }
-    for (int j = n > nf ? n - nf : 0; j < n && S.abort; j++) mbar_wait(&S.ffull[j % nf], (j / nf) & 1, err);
   } else if (tid == 128 * kGroups) {
     // products: one thread, its instructions are the step's serial part (with the loads and their waits in the same
     // thread, and slots counted by divisions, it set the time: 480 us per column at 7380 x 1000)
@@ -354,6 +355,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (!mbar_wait(&S.done, 0, err)) S.abort = 1;
   }
   __syncthreads();
+  // a wait gave up, perhaps after the last image was issued: let the images land before the CTA ends (bounded)
+  if (S.abort)
+    for (int j = loaded > nf ? loaded - nf : 0; j < loaded; j++) mbar_wait(&S.ffull[j % nf], (j / nf) & 1, err);
   tc_fence_after();
   if (warp < 4 && !S.abort && __all_sync(0xffffffffu, mbar_wait(&S.done, 0, err))) {
     tc_fence_after();
