@@ -580,11 +580,13 @@ __device__ __forceinline__ void fx_rmw_reg(u32* dst, const u32* x, const u32* y,
 // fx_rmw with both operands bounded by compile-time tops (|x| top <= LX, |y| top <= LY) and LF fraction words:
 // both in registers, every column sum unrolled over its exact term range (columns LF - 2 .. LX + LY, zero
 // beyond the actual tops), so no multiply-add is predicated away.  The same result as fx_rmw.
+// sh (0 or 1): |x| is taken times 2^(32 sh), i.e. the product is that of LF_ - sh fraction words, column for column.
 template <int LF_, int LX, int LY>
-__device__ __forceinline__ void fx_rmw_reg2(u32* dst, const u32* x, const u32* y, bool add, int WL) {
+__device__ __forceinline__ void fx_rmw_reg2(u32* dst, const u32* x, const u32* y, bool add, int WL, int sh = 0) {
   u32 xr[LX + 1], yr[LY + 1];
+  xr[0] = sh ? 0u : x[0];
 #pragma unroll
-  for (int i = 0; i <= LX; i++) xr[i] = x[i];
+  for (int i = 1; i <= LX; i++) xr[i] = x[i - sh];
 #pragma unroll
   for (int i = 0; i <= LY; i++) yr[i] = y[i];
   u32 c0 = 0, c1 = 0, c2 = 0, cy = 0;
@@ -627,6 +629,38 @@ __device__ __forceinline__ void fx_rmw_reg2(u32* dst, const u32* x, const u32* y
   emit(c0);                                              // columns LX + LY + 1, + 2: no new terms
   emit(c1);
   while (cy && w < WL) emit(0);
+}
+
+// fx_rmw of a well scaled tile's operands, |x| < 1 and |y| < 2^32 (tops below LF and up to LF), for 3 to 40 fraction
+// words: fx_rmw_reg2 at LF rounded up to even.  The inverse's products, in its only loop, so the switch is uniform.
+constexpr int kTightMin = 3, kTightMax = 40;
+__device__ __forceinline__ void fx_rmw_tight(u32* dst, const u32* x, const u32* y, bool add, int WL, int LF) {
+  const int sh = LF & 1;
+  switch (LF + sh) {
+#define SDPV_TIGHT(n) \
+  case n:             \
+    return fx_rmw_reg2<n, n - 1, n>(dst, x, y, add, WL, sh);
+    SDPV_TIGHT(4)
+    SDPV_TIGHT(6)
+    SDPV_TIGHT(8)
+    SDPV_TIGHT(10)
+    SDPV_TIGHT(12)
+    SDPV_TIGHT(14)
+    SDPV_TIGHT(16)
+    SDPV_TIGHT(18)
+    SDPV_TIGHT(20)
+    SDPV_TIGHT(22)
+    SDPV_TIGHT(24)
+    SDPV_TIGHT(26)
+    SDPV_TIGHT(28)
+    SDPV_TIGHT(30)
+    SDPV_TIGHT(32)
+    SDPV_TIGHT(34)
+    SDPV_TIGHT(36)
+    SDPV_TIGHT(38)
+    SDPV_TIGHT(40)
+#undef SDPV_TIGHT
+  }
 }
 
 // fx_rmw with only the first operand bounded (top <= LFT, kept in registers) and the second read from shared
@@ -1083,6 +1117,7 @@ __global__ void __launch_bounds__(kThreadsS) trinv_tiles_k(const u32* __restrict
   uint8_t* ls = xt + 528;                                        // signs, tops of the columns of L (2 x 32)
   uint8_t* lt = ls + 64;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool tight = !GLOBAL && LF >= kTightMin && LF <= kTightMax && WL > ((LF + 1) & ~1);   // (registers; words read)
   const u32* LG = Lt + (size_t)blockIdx.x * BT * BT * WL;
   const u32* RI = RINV + (size_t)blockIdx.x * BT * WL;
   u32* XG = X + (size_t)blockIdx.x * BT * BT * WL;
@@ -1132,12 +1167,12 @@ __global__ void __launch_bounds__(kThreadsS) trinv_tiles_k(const u32* __restrict
       u32* dst = Xm + (size_t)tri(i, k) * WP;
       const u32 *xl = Lc + (size_t)i * WP, *yx = Xm + (size_t)e * WP;
       const bool add = lsj[i] == xs[e];
-      // tops as tight as a well scaled tile has them (|l_ij| < 1, |x_jk| < 2^32): the multiplier sets a row's time
-      // (9.8 of 13 thousand cycles at 537 multiply-adds a product), and these take 402
-      if (LF == 26 && ltj[i] <= 25 && xt[e] <= 26)
-        fx_rmw_reg2<26, 25, 26>(dst, xl, yx, add, WL);
-      else if (LF == 24 && ltj[i] <= 23 && xt[e] <= 24)
-        fx_rmw_reg2<24, 23, 24>(dst, xl, yx, add, WL);
+      // tops as tight as a well scaled tile has them (|l_ij| < 1, |x_jk| < 2^32): the multiplier sets a row's time (9.8 of
+      // 13 thousand cycles at L = 26 with 537 multiply-adds a product; these take 402), and fx_rmw's dynamic range keeps
+      // it waiting: inverse of one tile at L = 4 / 8 / 16 / 20 / 25 / 28 / 34 / 40 from 139 / 185 / 291 / 351 / 435 / 490 /
+      // 633 / 758 us to 95 / 107 / 143 / 160 / 195 / 207 / 275 / 323; 197 at 26, as with products for that width alone
+      if (tight && ltj[i] < LF && xt[e] <= LF)
+        fx_rmw_tight(dst, xl, yx, add, WL, LF);
       else if (LF == 26 && ltj[i] <= 26 && xt[e] <= 30)
         fx_rmw_reg2<26, 26, 30>(dst, xl, yx, add, WL);
       else if (LF == 24 && ltj[i] <= 24 && xt[e] <= 28)
