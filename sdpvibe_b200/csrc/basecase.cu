@@ -1173,9 +1173,9 @@ __global__ void __launch_bounds__(kThreadsS) trinv_tiles_k(const u32* __restrict
       // 633 / 758 us to 95 / 107 / 143 / 160 / 195 / 207 / 275 / 323; 197 at 26, as with products for that width alone
       if (tight && ltj[i] < LF && xt[e] <= LF)
         fx_rmw_tight(dst, xl, yx, add, WL, LF);
-      else if (LF == 26 && ltj[i] <= 26 && xt[e] <= 30)
+      else if (LF == 26 && ltj[i] <= 26 && xt[e] <= 30 && WL > 30)      // (words up to 30 are read)
         fx_rmw_reg2<26, 26, 30>(dst, xl, yx, add, WL);
-      else if (LF == 24 && ltj[i] <= 24 && xt[e] <= 28)
+      else if (LF == 24 && ltj[i] <= 24 && xt[e] <= 28 && WL > 28)
         fx_rmw_reg2<24, 24, 28>(dst, xl, yx, add, WL);
       else if (LF == 26 && ltj[i] <= 26)
         fx_rmw_lreg<26>(dst, xl, yx, xt[e], add, WL);

@@ -75,6 +75,21 @@ def test_inverse_around_the_unrolled_products(L, extra):
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("L,extra", [(24, 2), (24, 4), (24, 5), (26, 2), (26, 4), (26, 5)])
+def test_inverse_with_few_words_above_the_point(L, extra):
+    """entries of the inverse over 2^32 in tiles of 2 to 5 words above the point: nothing past an entry's words is read"""
+    rng = np.random.default_rng(L + extra)
+    WL, one = L + extra, 1 << (32 * L)
+    Lw, RR = np.zeros((1, 32, 32, WL), np.uint32), np.zeros((1, 32, WL), np.uint32)
+    for i in range(32):
+        RR[0, i] = _words((one << 33) + int.from_bytes(rng.bytes(4 * L), "little"), WL) if i == 0 else _words(one, WL)
+        for j in range(i):
+            Lw[0, i, j] = _words(int.from_bytes(rng.bytes(4 * L), "little") % one >> 40, WL)
+        Lw[0, i, i] = _words(one, WL)
+    got, want = _invert(Lw, RR, WL, L)
+    assert np.array_equal(got, want)
+
+
 @pytest.mark.parametrize("L", [4, 7, 16, 24, 27, 34, 40])
 @pytest.mark.parametrize("ill", [False, True])
 def test_tiles_by_limb_count(L, ill):
