@@ -92,7 +92,9 @@ int sdpv_mpf_mul(int L, int64_t n, const int32_t* A, const int64_t* eA, const in
 int sdpv_mpf_add(int L, int64_t n, const int32_t* A, const int64_t* eA, const int32_t* Bm, const int64_t* eB,
                  int sgn, int32_t* O, int64_t* eO, void* stream);
 /* ---------------------------------------------------------------- launch-shape knobs (autotuner)
- * Results never depend on them.  SDPV_TUNE_CRT_CTAS: CRT CTAs per SM (1..4, default 3);
+ * Results never depend on them.  SDPV_TUNE_CRT_CTAS: CTAs per SM of the one-tile CRT, which takes calls of at most
+ * two 128-entry tiles per SM, and all with over 128 moduli (one CTA per SM there): 1..4, default 3; two and more
+ * differ in no call;
  * SDPV_TUNE_NARROW_MAX: residue-GEMM narrow items when one side has at most this many rows (0 = never,
  * else a multiple of 16 up to 64; default 64); SDPV_TUNE_PACK_MAX: small blocks packed several to a tile
  * when both sides have at most this many rows (0 = never, multiple of 16 up to 64; default 64);

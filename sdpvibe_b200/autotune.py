@@ -6,8 +6,9 @@ items; every choice gives the same bits.
     python -m sdpvibe_b200.autotune [--reps 5]      (on the GPU the table is for)
 
 Knobs and their shapes:
-  crt_ctas    CTAs per SM of the CRT: crt_block of the triangular solves' products (90 x 32 x 1000
-              entries), crt_norm of the Gram step (274 x 274)
+  crt_ctas    CTAs per SM of the one-tile CRT, which takes calls of at most two 128-entry tiles per SM: crt_block of
+              30000 entries (235 tiles), crt_norm of 22500 (176); larger calls go four tiles to an SM whatever
+              the knob says
   narrow_max  short-side limit of the narrow residue-GEMM items: the solves' block products
               (90 x 32 x 1000, K 32; 30 x 64 x 1000, K 64; 131 x 96 x 8, K 64)
   pack_max    block size limit for packing small blocks into one GEMM tile: the Cholesky recursion of
@@ -38,7 +39,7 @@ from . import _lib
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 TABLE = os.path.join(HERE, "tuning_b200.json")
-KNOBS = {"crt_ctas": (0, [1, 2, 3, 4]), "narrow_max": (1, [0, 32, 48, 64]), "pack_max": (2, [0, 32, 64]),
+KNOBS = {"crt_ctas": (0, [1, 2]), "narrow_max": (1, [0, 32, 48, 64]), "pack_max": (2, [0, 32, 64]),
          "res_warps": (3, [8, 16]), "moduli_group": (4, [16, 8, 4, 1])}
 
 
@@ -140,12 +141,12 @@ def tune(reps=5, L=26):
     R = lib_ctx(L)
     rng = np.random.default_rng(0)
     m = torch.tensor(R.mods, dtype=torch.int64, device="cuda")[:, None, None]
-    acc_s = (torch.randint(0, 1 << 30, (R.n, 2880, 1000), device="cuda") % m).to(torch.int16)
-    acc_g = (torch.randint(0, 1 << 30, (R.n, 274, 274), device="cuda") % m).to(torch.int16)
-    z274 = torch.zeros(274, dtype=torch.int64, device="cuda")
+    acc_s = (torch.randint(0, 1 << 30, (R.n, 200, 150), device="cuda") % m).to(torch.int16)
+    acc_g = (torch.randint(0, 1 << 30, (R.n, 150, 150), device="cuda") % m).to(torch.int16)
+    z150 = torch.zeros(150, dtype=torch.int64, device="cuda")
     cases = {
-        "crt_ctas": [lambda: R.crt_block(acc_s, 1000, 0, 1000, 2880),
-                     lambda: R.crt_norm(acc_g, 274, 0, 274, 274, z274, z274, L - 1)],
+        "crt_ctas": [lambda: R.crt_block(acc_s, 150, 0, 150, 200),
+                     lambda: R.crt_norm(acc_g, 150, 0, 150, 150, z150, z150, L - 1)],
         "narrow_max": [_gemm_case(R, 90, 32, 1000, 32, rng), _gemm_case(R, 30, 64, 1000, 64, rng),
                        _gemm_case(R, 131, 96, 8, 64, rng)],
         "pack_max": [_gemm_case(R, 106, 32, 32, 32, rng), _gemm_case(R, 131, 64, 32, 64, rng),

@@ -472,15 +472,10 @@ int launch_crt_t(const sdpv_ctx* c, const int16_t* acc, i64 ldg, i64 N, i64 j0, 
   if (nslot > nchunk) nslot = nchunk;
   u32 tcols = 128;
   while ((int)tcols < kDig * nchunk) tcols *= 2;
-  // CTAs per SM: what shared memory and TMEM hold, at most the tuned count (and no more may become resident
-  // than TMEM serves)
-  size_t smem = fixed + nslot * chunk;
-  const int by_tmem = 512 / (int)tcols;
+  // CTAs per SM: what shared memory holds (three with one digit chunk, two with two, one with two K tiles: never more
+  // than TMEM's 512 columns serve), at most the tuned count.  With one K tile the calls have at most two tiles per SM.
+  const size_t smem = fixed + nslot * chunk;
   int per_sm = (int)((228 * 1024) / (smem + 1024));
-  if (per_sm > by_tmem) {
-    per_sm = by_tmem;
-    smem = (228 * 1024) / (by_tmem + 1);
-  }
   const int tuned = sdpv::tune(SDPV_TUNE_CRT_CTAS);
   if (per_sm > tuned) per_sm = tuned;
   if (per_sm < 1) per_sm = 1;
