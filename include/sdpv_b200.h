@@ -337,7 +337,7 @@ int sdpv_grp_copy(int32_t* const* src_host, const int64_t* src_planes_host, int 
  * arena blocks: desc (40 int64 each: out arena, out base, out ld, base arena or -1, base base, base ld, rows,
  * cols, nsrc <= 7, then per source CRT entry base, sign, shift constant, exponent index or -1):
  * out = base + sum sign round(W / 2^(cst - xe[idx])) mod 2^(32L) -- btrsm_right's and bchol's rounded
- * products and exact differences (sdpvibe/batched.py:274-305, 82-92). */
+ * products and exact differences (sdpvibe/batched.py:274-305, 82-92).  L <= 144 (the tile kernels take L <= 72). */
 int sdpv_grp_finish_fixed(const int32_t* Wd, int W, int64_t Ntot, int64_t w, int32_t* const* ar_host,
                           const int64_t* planes_host, int nar, int L, const int64_t* xe, const int64_t* desc,
                           int64_t ndesc, void* stream);
@@ -346,18 +346,19 @@ int sdpv_grp_finish_fixed(const int32_t* Wd, int W, int64_t Ntot, int64_t w, int
  * ncols <= 32, eA constant, eA index or -1, B row tile, mode, base row tile0, destination row tile0); the
  * group's column exponent from its rows' maximal bit length, then store (mode 0) or the aligned difference /
  * sum with the base rows (modes 1 / 2) -- btrsm_left's leaf, update and badd 'align' (sdpvibe/batched.py:
- * 200-231, 313-352, 55-92). */
+ * 200-231, 313-352, 55-92).  L <= 128. */
 int sdpv_grp_solve_round(const int32_t* Wd, const int64_t* bl, int W, int64_t Ntot, int64_t w, int32_t* P,
                          int64_t Pplane, int64_t* Pe, int64_t m, int L, const int64_t* xe, const int64_t* desc,
                          int64_t ndesc, void* stream);
 
 /* Common column exponents of a tree node's row tiles: desc (4 int64 each: row tile0, row tiles, column0,
- * ncols <= 32); both halves re-rounded to the larger exponent (sdpvibe/batched.py:332-335, 349-352). */
+ * ncols <= 32); both halves re-rounded to the larger exponent (sdpvibe/batched.py:332-335, 349-352).  L <= 440. */
 int sdpv_grp_merge(int32_t* P, int64_t Pplane, int64_t* Pe, int64_t m, int L, const int64_t* desc, int64_t ndesc,
                    void* stream);
 
 /* Diagonal tiles of the factor arena (entry bases fbase, exponent e) -> wide fixed point (ntiles, 32, 32, WL)
- * at exponent -32 LF, zero above the diagonal (sdpvibe/batched.py:250). */
+ * at exponent -32 LF, zero above the diagonal (sdpvibe/batched.py:250).  L + WL < 440 (the tile kernels take WL <= 96,
+ * sdpv_grp_tile_narrow WL <= 219). */
 int sdpv_grp_tile_widen(const int32_t* Fa, int64_t Fplane, int L, int64_t e, int WL, int LF, const int64_t* fbase,
                         int64_t ntiles, uint32_t* out, void* stream);
 

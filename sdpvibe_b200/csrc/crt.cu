@@ -19,9 +19,10 @@
 // What bounds it: instruction issue of the pre-pass (about 11 instructions per residue) and, for a few tiles,
 // the latency of one tile's phases.  Both digits of y in one contraction halve the TMEM columns and take the
 // digit recombination and k Md out of the epilogue.  Measured (B200, against two signed digit products in four
-// waited-for chunks with the words in local memory): 158760 entries at 116 moduli 130 -> 68 us, 65536 at 104
-// 48 -> 30 us, 1000 entries 37 -> 15 us; crt_block of 1024 entries 22 -> 15 us.  Two CTAs per SM, one tile each
-// (102 KB at 116 moduli): the table twice on the SM costs less than two tiles waiting for one another.
+// waited-for chunks with the words in local memory): 1000 entries at 116 moduli 37 -> 15 us, crt_block of 1024 entries
+// 22 -> 15 us; over 128 moduli, whose table passes through the SM once per tile, 160000 entries at L = 34 349 -> 144 us
+// and at 58 603 -> 232.  Calls of at most two tiles per SM run as CTAs of one tile (two per SM up to 128 moduli, 102 KB
+// each at 116); larger ones with at most 128 moduli take crt4_kernel below.
 #include "common.cuh"
 #include "crt_reduce.h"
 #include "mpcol.cuh"
@@ -43,8 +44,8 @@ struct CrtHead {
   int abort;
 };
 
-// Four digit columns as one word's contribution.  WIDE: z0 + 2^8 z1 may exceed 32 bits (z <= n 381 255, so for
-// n > 168 as 257 n 381 255 >= 2^32).
+// Four digit columns as one word's contribution.  WIDE: z0 + 2^8 z1 may exceed 32 bits (z <= n 381 255, and
+// 257 n 381 255 >= 2^32 from n = 173 on; taken from 169 on).
 template <bool WIDE>
 __device__ __forceinline__ u64 digit_word(const u32* z) {
   if (WIDE) return ((u64)z[0] + ((u64)z[1] << 8)) + ((((u64)z[2]) + ((u64)z[3] << 8)) << 16);
@@ -275,8 +276,8 @@ __global__ void __launch_bounds__(kThreads, 2)
 // The same for calls of many tiles with n <= 128 (one or two digit chunks): kWide tiles at a time on an SM, each worked
 // by its own four warps, which share one copy of the table.  TMEM then holds one chunk per tile, so the chunks run
 // one after the other, the first one's words waiting in registers while the second's product still reads Y.
-// Measured against two one-tile CTAs per SM (8 warps, latency-bound): 158760 entries at 116 moduli 68 -> 54 us,
-// 65536 at 104 30 -> 22, the 34 calls of a 600-block Cholesky and solve 5.8 -> 4.1 ms.
+// Measured against two one-tile CTAs per SM (8 warps, latency-bound): 158760 entries at 116 moduli 68 -> 54 us
+// (130 before the one contraction), 65536 at 104 30 -> 22, the 34 calls of a 600-block Cholesky and solve 5.8 -> 4.1 ms.
 constexpr int kWide = 4;
 struct Crt4Head {
   u64 full, done[kWide];

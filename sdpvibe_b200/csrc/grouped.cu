@@ -25,7 +25,7 @@
 namespace {
 
 constexpr int kArenas = 4;
-constexpr int kLMax = 128;                 // limbs of an intermediate kept in registers / local memory
+constexpr int kLMax = 128;                 // most limbs of a solve's right-hand sides (shared-memory columns of 128 threads)
 constexpr int kMaxSrc = 7;                 // rounded products summed into one destination by grp_finish_fixed
 
 struct Arenas {
@@ -124,15 +124,15 @@ __global__ void __launch_bounds__(256) grp_copy_kernel(Arenas src, int32_t* __re
 // then per source: CRT entry base, sign (+1 / -1), shift constant, exponent index (-1: none).  Entry (r, c):
 //   out = base + sum_i sign_i round(W_i[r][c] / 2^s_i) mod 2^(32 L),  s_i = cst_i - xe[idx_i]
 // where W_i[r][c] is the CRT value (W words, planes Ntot apart) at entry crt_base_i + r * w + c.  Eight CTAs per
-// descriptor (grid y), one entry per thread for a 32 x 32 block.  Only the L + 2 words that the rounding reads
-// are staged; the next source is in flight while one is added (the word-by-word loads of a plain loop had set
-// the time: 20 us a launch of few tiles, with 32 of them per factorisation of 9 tile columns).
+// descriptor (grid y), one entry per thread for a 32 x 32 block.  Only the L + 2 words that the rounding reads and the
+// sign word are staged; the next source is in flight while one is added (the word-by-word loads of a plain loop had
+// set the time: 20 us a launch of few tiles, with 32 of them per factorisation of 9 tile columns).
 constexpr int kFinT = 128;
 __global__ void __launch_bounds__(kFinT) grp_finish_fixed_kernel(const int32_t* __restrict__ Wd, int W, i64 Ntot, i64 w,
                                                                  Arenas ar, int L, const i64* __restrict__ xe,
                                                                  const i64* __restrict__ desc) {
   extern __shared__ u32 cols[];
-  u32* sum = cols + threadIdx.x;                        // L words, then two source columns of L + 2 words
+  u32* sum = cols + threadIdx.x;                        // L words, then two source columns of L + 3 words
   u32* buf = sum + L * kFinT;
   const i64* d = desc + 40 * (i64)blockIdx.x;
   const int oid = (int)d[0], bid = (int)d[3], rows = (int)d[6], ncol = (int)d[7];
@@ -146,23 +146,22 @@ __global__ void __launch_bounds__(kFinT) grp_finish_fixed_kernel(const int32_t* 
     int32_t* op = ar.p[oid] + obase + (i64)r * old_ + c;
     const i64 oplane = ar.plane[oid];
     // words b0 .. of source i: those from the rounding bit's word up to word q + L, and the top (sign) word last
-    auto issue = [&](int i, int& s, int& b0, int& cnt) {
+    auto issue = [&](int i, int& s, int& b0) {
       const i64* si = d + 9 + 4 * i;
       s = clamp_shift(si[2] - (si[3] >= 0 ? xe[si[3]] : 0), W, L);
       const int q = s >> 5;
       b0 = q - 1 > 0 ? (q - 1 < W - 1 ? q - 1 : W - 1) : 0;
       const int e = q + L + 1 < W ? (q + L + 1 > b0 ? q + L + 1 : b0) : W;    // [b0, e)
-      cnt = e - b0;
       const int32_t* src = Wd + si[0] + (i64)r * w + c;
       u32* dst = buf + (i & 1) * (L + 3) * kFinT;
-      stage_col(dst, kFinT, src + (i64)b0 * Ntot, Ntot, cnt);
+      stage_col(dst, kFinT, src + (i64)b0 * Ntot, Ntot, e - b0);
       cp_async4(dst + (L + 2) * kFinT, src + (i64)(W - 1) * Ntot, 4u);
     };
-    int s0 = 0, b0 = 0, n0 = 0, s1 = 0, b1 = 0, n1 = 0;
-    if (ns > 0) issue(0, s0, b0, n0);
+    int s0 = 0, b0 = 0, s1 = 0, b1 = 0;
+    if (ns > 0) issue(0, s0, b0);
     cp_async_commit();
     for (int i = 0; i < ns; i++) {
-      if (i + 1 < ns) issue(i + 1, s1, b1, n1);
+      if (i + 1 < ns) issue(i + 1, s1, b1);
       cp_async_commit();
       cp_async_wait<1>();
       const u32* col = buf + (i & 1) * (L + 3) * kFinT;
@@ -181,7 +180,6 @@ __global__ void __launch_bounds__(kFinT) grp_finish_fixed_kernel(const int32_t* 
       }
       s0 = s1;
       b0 = b1;
-      n0 = n1;
     }
     if (ns == 0) {
       cp_async_wait<0>();

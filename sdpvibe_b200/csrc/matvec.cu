@@ -1,6 +1,6 @@
 // C = A^T B for a long, wide A (K, M) and a few columns B (K, N): the residual products of the solver (B^T x).
 //
-// A residue product decomposes every entry of A into 2 n residue bytes to use each once: 637 of 1420 us for 7380 x
+// A residue product decomposes every entry of A into 2 n residue bytes to use each once: 637 of 1500 us for 7380 x
 // 1000 by one column at L = 26, against 127 us that reading A takes.  Here A's entries meet the column directly on
 // the tensor cores.  With numbers as signed base-256 digits (a + 0x8080..80 per byte, then each byte less 128),
 //   c_i = sum_k a_ik x_k = sum_t 256^t sum_k sum_j a_ik[j] x_k[t - j],
@@ -15,10 +15,10 @@
 //     streams the Toeplitz operands (bulk copies) and issues the products; the int32 sums of the range go to
 //     the workspace.
 //   * mv_finish: sums over the ranges, carries, renormalisation (mpcol.cuh).
-// The sums are exact, so the result is that of the residue product bit for bit.  7380 x 1000 by one column: 1420 ->
-// 375 us (mv_main 319), by two (A rounded once for both) 494.  What bounds mv_main: the rounding's instructions and
-// waits (251 us without it) over about 105 KB of shared-memory traffic per k (820 cycles).  Three groups of aligners
-// with three rows of A staged each: two groups 381 us, four with two rows 321 (shared memory holds no more).
+// The sums are exact, so the result is that of the residue product bit for bit.  7380 x 1000 by one column: 1503-1530 ->
+// 376-426 us on several boxes (mv_main 319), by two (A rounded once for both) 494.  What bounds mv_main: the rounding's
+// instructions and waits (251 us without it) over about 105 KB of shared-memory traffic per k (820 cycles).  Three groups
+// of aligners with three rows of A staged each: two groups 381 us, four with two rows 321 (shared memory holds no more).
 #include <cstring>
 
 #include "common.cuh"

@@ -8,7 +8,9 @@
 // the same operations on u32 arrays of the entry in local memory: product of 605160 entries at L = 26 291 -> 84
 // us (2.4 TB/s of operands and result; the short product's multiply-adds and its 8 shared-memory reads per 16 of
 // them are the larger part), sum of 150001 at L = 50 142 -> 37 us (2.5 TB/s; the passes of one CTA are in
-// sequence and shared memory holds four CTAs of 128 such entries).
+// sequence and shared memory holds four CTAs of 128 such entries).  Wider numbers leave fewer CTAs per SM (one of
+// products at 128 and 160 limbs) and still gain: 200000 entries at L = 64 / 100 / 160 products 611 -> 119, 2070 -> 280,
+// 6941 -> 780 us, sums 326 -> 62, 594 -> 114, 1024 -> 229.
 #pragma once
 #include "common.cuh"
 

@@ -59,3 +59,8 @@ def test_count_beyond_the_buffer():
     from sdpvibe_b200.sdp_io import decode_bigfloats
     with pytest.raises(ValueError):
         decode_bigfloats(b"\x01" * 64, 0, 1 << 36, 18, 26)
+
+
+def test_round_trip_zeros_above_the_limit():
+    """zeros among records of over 1 MiB (9000 records with a third of them zero stay below it)"""
+    test_round_trip(15000, True)
