@@ -16,8 +16,9 @@
 //     products are done with it) and renormalises from there (mpcol.cuh).
 // No intermediate leaves the SM; one launch replaces crt_pre + digit GEMM + crt_carry + normalize.
 //
-// What bounds it: instruction issue of the pre-pass (about 11 instructions per residue) and, for a few tiles,
-// the latency of one tile's phases.  Both digits of y in one contraction halve the TMEM columns and take the
+// What bounds it: latency.  A one-tile CTA's four warps go through its phases one after the other (issue active in 21 %
+// of the cycles with 235 tiles); four tiles on an SM wait for the residues' loads (49 %), the pre-pass's instructions
+// (about 11 per residue) being the larger part of what is issued.  Both digits of y in one contraction halve the TMEM columns and take the
 // digit recombination and k Md out of the epilogue.  Measured (B200, against two signed digit products in four
 // waited-for chunks with the words in local memory): 1000 entries at 116 moduli 37 -> 15 us, crt_block of 1024 entries
 // 22 -> 15 us; over 128 moduli, whose table passes through the SM once per tile, 160000 entries at L = 34 349 -> 144 us
